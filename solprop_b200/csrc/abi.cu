@@ -296,8 +296,9 @@ struct sp_workspace {
   DevBuf<double> raman_undamped, raman_weights;
   DevBuf<double> stat_power, stat_out, stat_weight;  // plane statistics, on first use
   DevBuf<double2> raman_spectrum;  // field-grid Raman: the damped kernel's spectrum (n_to + 1)
-  DevBuf<float2> raman_spectrum32;  // the envelope products' mixed form: the spectra scaled, complex64
-  DevBuf<int> raman_scale;          // ... and their powers of two
+  DevBuf<int> raman_scale;         // the envelope products' mixed form: the spectra's powers of two
+  // the envelope products' nodes: the spectra and twiddles in the register transform's order
+  DevBuf<double2> raman_table, outer_twiddles, inner_twiddles;
   DevBuf<double2> env_scratch;      // the envelope products' FP64 rows above 8192 samples: 1.5 n_to per row
   DevBuf<double2> raman_scratch;    // ... and the Raman kernel's spectra
   DevBuf<ChannelTableT<double>> channels;  // a mixture's plasma channels (rate_coeff holds their tables)
@@ -315,7 +316,7 @@ struct sp_workspace {
     DevBuf<float> t_window, t_window_d, synthesis, projection, rate_coeff, taps, proj;
     DevBuf<float> node_field, node_streams;
     DevBuf<ChannelTableT<float>> channels;
-    DevBuf<float2> env_twiddles;
+    DevBuf<float2> env_twiddles, raman_table, outer_twiddles, inner_twiddles;
   } f32;
   DevBuf<unsigned char> active, norm;
   DevBuf<StageScalarsDev> stage;   // kStageSlots slots
@@ -709,13 +710,18 @@ static EnvModalArgsT<R> env_modal_args(const sp_workspace* ws, const double2* la
   ea.raman_kernels = P.raman_kernels;
   if constexpr (sizeof(R) == 8) {
     ea.twiddles_r = ws->env_twiddles.p;
+    ea.raman_table = ws->raman_table.p;
+    ea.outer_twiddles = ws->outer_twiddles.p;
+    ea.inner_twiddles = ws->inner_twiddles.p;
     ea.node_field = ws->node_field.p;
     ea.node_streams = ws->node_streams.p;
     ea.projected = ws->proj.p;
     ea.spectra = ws->spectra.p;
   } else {
     ea.twiddles_r = ws->f32.env_twiddles.p;
-    ea.raman_spectrum32 = ws->raman_spectrum32.p;
+    ea.raman_table = ws->f32.raman_table.p;
+    ea.outer_twiddles = ws->f32.outer_twiddles.p;
+    ea.inner_twiddles = ws->f32.inner_twiddles.p;
     ea.raman_scale = ws->raman_scale.p;
     ea.node_field = ws->f32.node_field.p;
     ea.node_streams = ws->f32.node_streams.p;
@@ -745,9 +751,9 @@ static void eval_source_envelope_gemm(sp_workspace* ws, const double2* lab, int 
       KernelTimer t(ws, SP_K_COLUMN);
       if (d.raman_enabled) {
         RamanArgs ra = raman_args(ws, slot);
-        ra.spectrum32 = ws->raman_spectrum32.p;
         ra.scale = ws->raman_scale.p;
         CUDA_CHECK(launch_raman_spectrum(ra, ws->stream));
+        CUDA_CHECK(launch_raman_table(ea, ws->f32.raman_table.p, ws->stream));
       }
       CUDA_CHECK(launch_env_nodes(ea, d.n_nodes, ws->stream));
     }
@@ -769,7 +775,10 @@ static void eval_source_envelope_gemm(sp_workspace* ws, const double2* lab, int 
   }
   {
     KernelTimer t(ws, SP_K_COLUMN);
-    if (d.raman_enabled) CUDA_CHECK(launch_raman_spectrum(raman_args(ws, slot), ws->stream));
+    if (d.raman_enabled) {
+      CUDA_CHECK(launch_raman_spectrum(raman_args(ws, slot), ws->stream));
+      if (d.n_to <= kMaxEnvelopeRowF64) CUDA_CHECK(launch_raman_table(ea, ws->raman_table.p, ws->stream));
+    }
     CUDA_CHECK(launch_env_nodes(ea, d.n_nodes, ws->stream));
   }
   {
@@ -1043,8 +1052,8 @@ static void build_workspace(sp_workspace* ws) {
   ws->norm_arrivals.alloc(1);
   ws->norm_arrivals.zero(s);
   ws->launches = 5;
-  if (ws->gemm && d.grid_kind == 1) {  // inverse, synthesis, (Raman spectrum,) nodes, projection, reduction,
-    ws->launches = 6 + (d.raman_enabled ? 1 : 0) + (ws->precision == SP_PRECISION_MIXED ? 2 : 0);  // forward,
+  if (ws->gemm && d.grid_kind == 1) {  // inverse, synthesis, (Raman spectrum, table,) nodes, projection, reduction,
+    ws->launches = 6 + (d.raman_enabled ? 2 : 0) + (ws->precision == SP_PRECISION_MIXED ? 2 : 0);  // forward,
                                                                   // output; the mixed form's two split passes
   } else if (ws->gemm) {  // inverse, synthesis, column, one projection per stream, forward, output
     const int per_product = ws->precision == SP_PRECISION_MIXED ? 2 : 1;  // (split,) product
@@ -1069,9 +1078,28 @@ static void build_workspace(sp_workspace* ws) {
     if (!P.raman_weights.empty()) ws->raman_weights.upload(P.raman_weights.data(), P.raman_weights.size(), s);
     if (d.raman_enabled && (d.grid_kind == 0 || ws->gemm))
       ws->raman_spectrum.alloc((size_t)P.raman_kernels * (d.n_to + 1));
-    if (d.raman_enabled && d.grid_kind == 1 && ws->gemm && ws->precision == SP_PRECISION_MIXED) {
-      ws->raman_spectrum32.alloc((size_t)P.raman_kernels * (d.n_to + 1));
-      ws->raman_scale.alloc(2);
+    if (d.raman_enabled && d.grid_kind == 1 && ws->gemm) {
+      // the nodes' register transform (FP64 rows above kMaxEnvelopeRowF64 take the long form)
+      std::vector<double2> outer, inner;
+      env_pair_twiddles(d.n_to, tw2, outer, inner);
+      const size_t table = (size_t)2 * P.raman_kernels * d.n_to;
+      if (ws->precision == SP_PRECISION_MIXED) {
+        auto narrow = [&](const std::vector<double2>& v, DevBuf<float2>& dst) {
+          std::vector<float2> f(v.size());
+          for (size_t m = 0; m < v.size(); ++m) f[m] = make_float2((float)v[m].x, (float)v[m].y);
+          dst.upload(f.data(), f.size(), s);
+          CUDA_CHECK(cudaStreamSynchronize(s));  // the host copy goes with this scope
+        };
+        narrow(outer, ws->f32.outer_twiddles);
+        narrow(inner, ws->f32.inner_twiddles);
+        ws->f32.raman_table.alloc(table);
+        ws->raman_scale.alloc(2);
+      } else if (d.n_to <= kMaxEnvelopeRowF64) {
+        ws->outer_twiddles.upload(outer.data(), outer.size(), s);
+        ws->inner_twiddles.upload(inner.data(), inner.size(), s);
+        CUDA_CHECK(cudaStreamSynchronize(s));  // the host copies go with this scope
+        ws->raman_table.alloc(table);
+      }
     }
     if (d.grid_kind == 1 && ws->gemm && d.n_to > kMaxEnvelopeRowF64) {
       // rows of FP64 too long for one CTA: the inverse transforms' (every column), and in the

@@ -11,15 +11,20 @@
 //   products       E = tau S a and P_m = sum W P / tau over the interleaved rows
 //                  (modal_gemm.cu), N = 2 n_to: FP64 products, or tcgen05 products of
 //                  three-part BF16 splits accumulated in FP32 in the mixed form
-//   k_env_nodes    one CTA per node: the Kerr cubic, the Raman convolution, the window g
+//   k_env_pairs    one CTA per two nodes: the Kerr cubic, the Raman convolutions, the window g
+//                  (k_env_kerr without Raman; k_env_nodes_long for FP64 rows of 16 384)
 //   k_env_forward  one CTA per modal column: fft of the projected row, cropped
 //
-// Every transform is the shared-memory radix-4 FFT of fft.cuh over the table
-// exp(-2 pi i m / (2 n_to)), m < n_to.  The inverse transform and the modal field are FP64
+// The columns' transforms are the shared-memory FFTs of fft.cuh over the table
+// exp(-2 pi i m / (2 n_to)), m < n_to; the nodes' the register FFT of fft_regs.cuh.  The inverse transform and the modal field are FP64
 // in both forms; the Kerr cubic, the Raman convolutions and the forward transform run in the
 // form's type R (FP32 in the mixed form).
+#include <algorithm>
+#include <type_traits>
+
 #include "fft.cuh"
 #include "fft_long.cuh"
+#include "fft_regs.cuh"
 #include "kernels.cuh"
 
 namespace sp {
@@ -28,27 +33,6 @@ namespace {
 
 constexpr double kEps0 = 8.8541878188e-12;  // vacuum permittivity (F/m), CODATA 2022, as solprop.constants
 constexpr int kEnvThreads = 1024;
-
-// X[k] = E_k + w^k O_k of a packed real transform of length 2 n (k in [0, n]); Z in
-// bit-reversed order, w = exp(-2 pi i k / 2n) = tw[k] (k < n), -1 at k = n
-template <class C>
-__device__ __forceinline__ C unpack_real(const C* Z, const C* tw, int k, int n, int log_n) {
-  using R = decltype(C{}.x);
-  const int kk = k == n ? 0 : k;
-  const int km = k == 0 ? 0 : (n - k == n ? 0 : n - k);
-  const C zk = Z[bitrev(kk, log_n)];
-  const C zm = cconj(Z[bitrev(km, log_n)]);
-  const C e = cscale(R(0.5), cadd(zk, zm));
-  const C o = cscale(R(0.5), mul_mi(csub(zk, zm)));
-  C w;
-  if (k < n) {
-    w = tw[k];
-  } else {
-    w.x = R(-1);
-    w.y = R(0);
-  }
-  return cadd(e, cmul(w, o));
-}
 
 template <class R>
 __global__ void __launch_bounds__(kEnvThreads) k_env_inverse(EnvModalArgsT<R> a) {
@@ -77,80 +61,7 @@ __global__ void __launch_bounds__(kEnvThreads) k_env_inverse(EnvModalArgsT<R> a)
     absorber[j] = to_c<cplx<R>>(B[bitrev((int)a.crop[j], a.log_n_to)]);
 }
 
-constexpr int kNodeThreads = 512;  // one radix-8 butterfly per thread at 4 096 samples
-constexpr int kMaxPairs = kMaxEnvelopeProducts / 2 / kNodeThreads + 1;
-
-// Y = H X on the packed spectrum of a real drive of length 2n, and the packing of the
-// inverse real transform, in place over the swizzled row: Z[j] (j < n, bit-reversed slots)
-// holds the forward transform of d(2m) + i d(2m + 1).  Pair (k, n - k) needs Z[k] and
-// Z[n - k] alone and gives Z'[k] and Z'[n - k] (k = 0 also makes bin n), so every thread
-// reads its pairs, the block meets, and the thread writes them back in natural order:
-//   X[k] = E_k + w^k O_k,  E_k = (Z[k] + Z*[n-k]) / 2,  O_k = -i (Z[k] - Z*[n-k]) / 2
-//   Z'[k] = E'_k + i O'_k, E'_k = (Y[k] + Y*[n-k]) / 2, O'_k = (Y[k] - Y*[n-k]) conj(w^k) / 2
-// with w = exp(-2 pi i / 2n) and the imaginary parts of Y[0] and Y[n] dropped.
-// The Raman convolution's arithmetic: FP64 in the FP64 form; FP32 in the mixed form, on the
-// kernel spectrum scaled by 2^scale (a molecular gas's SI spectrum, about 1e-55, lies below
-// FP32's range; the scale is taken back out in FP64)
-template <class R>
-__device__ __forceinline__ const cplx<R>* spectrum_table(const EnvModalArgsT<R>& a) {
-  if constexpr (sizeof(R) == 8) return a.twiddles;
-  else return a.twiddles_r;
-}
-template <class R>
-__device__ __forceinline__ const cplx<R>* kernel_spectrum(const EnvModalArgsT<R>& a, int kernel) {
-  if constexpr (sizeof(R) == 8) return a.raman_spectrum + (size_t)kernel * (a.n_to + 1);
-  else return a.raman_spectrum32 + (size_t)kernel * (a.n_to + 1);
-}
-template <class R>
-__device__ __forceinline__ double spectrum_unscale(const EnvModalArgsT<R>& a, int kernel, double v) {
-  if constexpr (sizeof(R) == 8) return v;
-  else return scalbn(v, -a.raman_scale[kernel]);
-}
-
-template <class C>
-__device__ __forceinline__ void spectrum_product(C* B, const C* __restrict__ H, const C* __restrict__ tw, int n,
-                                                 int log_n) {
-  using T = decltype(C{}.x);
-  C za[kMaxPairs], zb[kMaxPairs];
-  int count = 0;
-  const T half = T(0.5);
-  for (int k = threadIdx.x; k <= n / 2; k += blockDim.x, ++count) {
-    const int km = k == 0 ? 0 : n - k;
-    const C a = B[row_slot<C>(bitrev(k, log_n))];
-    const C b = B[row_slot<C>(bitrev(km, log_n))];
-    if (k == 0) {
-      // X[0] = Re Z0 + Im Z0, X[n] = Re Z0 - Im Z0 (both real); Y's imaginary parts dropped;
-      // Z'[0] = (Y0 + Yn) / 2 + i (Y0 - Yn) / 2
-      C x0, xn;
-      x0.x = a.x + a.y;
-      x0.y = T(0);
-      xn.x = a.x - a.y;
-      xn.y = T(0);
-      const T y0 = cmul(H[0], x0).x, yn = cmul(H[n], xn).x;
-      za[count].x = half * (y0 + yn);
-      za[count].y = half * (y0 - yn);
-      zb[count] = za[count];
-      continue;
-    }
-    const C e = cscale(half, cadd(a, cconj(b)));
-    const C o = cscale(half, mul_mi(csub(a, cconj(b))));
-    const C wk = tw[k], wm = tw[km];
-    const C xk = cadd(e, cmul(wk, o));
-    // X[n - k]: E_{n-k} = conj(E_k), O_{n-k} = -i (Z[n-k] - Z*[k]) / 2
-    const C om = cscale(half, mul_mi(csub(b, cconj(a))));
-    const C xm = cadd(cconj(e), cmul(wm, om));
-    const C yk = cmul(H[k], xk), ym = cmul(H[km], xm);
-    za[count] = cadd(cscale(half, cadd(yk, cconj(ym))), mul_pi(cscale(half, cmul(csub(yk, cconj(ym)), cconj(wk)))));
-    zb[count] = cadd(cscale(half, cadd(ym, cconj(yk))), mul_pi(cscale(half, cmul(csub(ym, cconj(yk)), cconj(wm)))));
-  }
-  __syncthreads();
-  count = 0;
-  for (int k = threadIdx.x; k <= n / 2; k += blockDim.x, ++count) {
-    B[row_slot<C>(k)] = za[count];
-    if (k != 0 && k != n / 2) B[row_slot<C>(n - k)] = zb[count];
-  }
-  __syncthreads();
-}
+constexpr int kNodeThreads = 512;
 
 // One sample t of a node's gated polarisation: with drive 0 the Kerr cubic and the first
 // convolution conv (already times eps0 rho) times the field; the later drives add
@@ -194,73 +105,175 @@ __device__ __forceinline__ void node_sample(const EnvModalArgsT<R>& a, const cpl
   }
 }
 
-// The nodes' responses, one CTA per node.  The Raman convolutions run in the form's type
-// (the mixed form's on a scaled spectrum, above).  With two field components (rows x, y of the node) the
-// Kerr cubic sums over them and the Raman response is the tensor one
-// (passes/responses.py:501-550): the trace drive |a_x|^2/2 + |a_y|^2/2 and, with a
-// traceless kernel, the difference and coherence drives, three convolutions u, v, w whose
-// symmetric matrix [[u + v, w], [w, u - v]] multiplies the field.  Each convolution is
-// added to the node's stream as it is formed (the first with the Kerr cubic), so the row
-// of shared memory is the transform's alone.
+// The nodes' responses without Raman: the gated Kerr cubic, sample by sample
 template <class R>
-__global__ void __launch_bounds__(kNodeThreads, 2) k_env_nodes(EnvModalArgsT<R> a) {
+__global__ void __launch_bounds__(256) k_env_kerr(EnvModalArgsT<R> a, int n_nodes) {
+  const double factor = a.kerr ? a.kerr_coefficient * a.stage->kerr_density : 0.0;
+  const int nc = a.n_components, n = a.n_to;
+  const size_t total = (size_t)n_nodes * n;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+    const size_t node = i >> a.log_n_to;
+    const cplx<R>* Ex = reinterpret_cast<const cplx<R>*>(a.node_field) + node * nc * n;
+    cplx<R>* Px = reinterpret_cast<cplx<R>*>(a.node_streams) + node * nc * n;
+    const int step = nc == 2 ? n : 0;
+    node_sample<R>(a, Ex, Ex + step, Px, Px + step, (int)(i & (n - 1)), 0.0, 0, nc, factor, R(a.kerr_self),
+                   R(a.kerr_conjugate));
+  }
+}
+
+// One sample of a node's gated polarisation with every convolution at hand: the Kerr cubic
+// c rho (s (sum |a|^2) a_p + q (sum a^2) a_p*) and the Raman matrix [[u + v, w], [w, u - v]]
+// (already times eps0 rho) times the field.  The cubic is formed in R and its SI coefficient
+// (about 1e-37 for a gas) applied in FP64, so that it never rounds to an FP32 subnormal.
+template <class R>
+__device__ __forceinline__ void node_output(const EnvModalArgsT<R>& a, int nc, double factor, double gate,
+                                            cplx<R> x, cplx<R> y, double u, double v, double w, cplx<R>& px,
+                                            cplx<R>& py) {
   using C = cplx<R>;
-  extern __shared__ __align__(16) unsigned char en_raw[];
-  const int n = a.n_to, node = blockIdx.x, nc = a.n_components;
-  C* B = reinterpret_cast<C*>(en_raw);  // a drive's transform, then its convolution's (swizzled slots)
-  const StageScalarsDev& st = *a.stage;
-  const C* Ex = reinterpret_cast<const C*>(a.node_field) + (size_t)node * nc * n;
-  const C* Ey = Ex + (nc == 2 ? n : 0);
-  C* Px = reinterpret_cast<C*>(a.node_streams) + (size_t)node * nc * n;
-  C* Py = Px + (nc == 2 ? n : 0);
-  const bool raman = a.raman_spectrum != nullptr;
-  const int drives = !raman ? 0 : (nc == 2 && a.raman_kernels == 2 ? 3 : 1);
-  // the Kerr coefficient times the density (about 1e-37 in SI units for a gas) is applied in
-  // FP64 to the cubic formed in R, so that it never rounds to an FP32 subnormal
-  const double factor = a.kerr ? a.kerr_coefficient * st.kerr_density : 0.0;
   const R self = R(a.kerr_self), conj = R(a.kerr_conjugate);
-  const double raman_scale = kEps0 * (a.raman_mixture ? 1.0 : st.raman_density);  // a mixture's are inside
-  const double inv_n = 1.0 / (double)n;
-  for (int dr = 0; dr < (drives > 0 ? drives : 1); ++dr) {
-    if (drives > 0) {
-      // the drive on [0, n), zero on [n, 2n), packed: B[m] = d(2m) + i d(2m + 1)
-      for (int m = threadIdx.x; m < n; m += blockDim.x) {
-        R v[2] = {R(0), R(0)};
-        if (2 * m < n) {
-          for (int q = 0; q < 2; ++q) {
-            const C x = Ex[2 * m + q];
-            const R xx = R(0.5) * (x.x * x.x + x.y * x.y);
-            if (nc == 1) {
-              v[q] = xx;
-            } else {
-              const C y = Ey[2 * m + q];
-              const R yy = R(0.5) * (y.x * y.x + y.y * y.y);
-              v[q] = dr == 0 ? xx + yy : dr == 1 ? xx - yy : R(2) * R(0.5) * (x.x * y.x + x.y * y.y);
+  R mod = x.x * x.x + x.y * x.y;
+  C sq = cmul(x, x);
+  if (nc == 2) {
+    mod += y.x * y.x + y.y * y.y;
+    sq = cadd(sq, cmul(y, y));
+  }
+  const double2 dx = to_d2(x), dy = to_d2(y);
+  const double2 kx = to_d2(cadd(cscale(self * mod, x), cscale(conj, cmul(sq, cconj(x)))));
+  const double rx = u + v;
+  px = to_c<C>(make_double2(gate * fma(factor, kx.x, fma(rx, dx.x, w * dy.x)),
+                            gate * fma(factor, kx.y, fma(rx, dx.y, w * dy.y))));
+  if (nc == 2) {
+    const double2 ky = to_d2(cadd(cscale(self * mod, y), cscale(conj, cmul(sq, cconj(y)))));
+    const double ry = u - v;
+    py = to_c<C>(make_double2(gate * fma(factor, ky.x, fma(ry, dy.x, w * dx.x)),
+                              gate * fma(factor, ky.y, fma(ry, dy.y, w * dx.y))));
+  }
+}
+
+// The nodes' responses with Raman, one CTA per two nodes A and B.  A convolution with a real
+// kernel takes two real drives as one complex row: the trace drives of A and B together
+// (drive |a|^2 / 2, or |a_x|^2 / 2 + |a_y|^2 / 2 of two field components), then, where the
+// tensor response has a traceless kernel, each node's difference |a_x|^2 / 2 - |a_y|^2 / 2
+// and coherence Re(a_x a_y*) (passes/responses.py:501-550).  The convolutions are linear on
+// the doubled, zero-padded grid (Row::convolve of fft_regs.cuh), the spectra stored in the
+// transform's bin order (k_raman_table), so that no spectrum is unpacked or reordered.  The
+// trace convolutions wait for the traceless ones in the last node's polarisation row, each
+// thread reading back what it wrote there before it writes the polarisation.
+//
+// What bounds it: the transforms' FP32 (FP64) issue and their exchanges through shared memory.
+// The whole row lies in the registers of one CTA (32 points per thread) and crosses shared
+// memory four times per convolution half, where a shared-memory transform of packed real
+// drives (one CTA per node) crossed it nine times and gathered bit-reversed pairs besides.
+// 16 384 nodes of two components, rows of 16 384, FP32: 33.0 -> 7 ms; 2 025 nodes, rows of
+// 8 192, FP64: 2.78 -> 1.0 ms.
+template <class R, int LOGN>
+__global__ void __launch_bounds__(regs::Row<cplx<R>, LOGN>::T, (sizeof(R) == 4 ? 512 : 256) / regs::Row<cplx<R>, LOGN>::T)
+    k_env_pairs(EnvModalArgsT<R> a, int n_nodes) {
+  using C = cplx<R>;
+  using Row = regs::Row<C, LOGN>;
+  constexpr int n = Row::N, T = Row::T, V = Row::V;
+  extern __shared__ __align__(16) unsigned char ep_raw[];
+  C* stash = reinterpret_cast<C*>(ep_raw);
+  R* plane = reinterpret_cast<R*>(stash + n);
+  const int nc = a.n_components, t0 = threadIdx.x;
+  const int first = 2 * blockIdx.x, count = min(2, n_nodes - first);
+  const StageScalarsDev& st = *a.stage;
+  const double factor = a.kerr ? a.kerr_coefficient * st.kerr_density : 0.0;
+  const double density = kEps0 * (a.raman_mixture ? 1.0 : st.raman_density);  // a mixture's are inside
+  const C* const field = reinterpret_cast<const C*>(a.node_field) + (size_t)first * nc * n + t0;
+  C* const stream = reinterpret_cast<C*>(a.node_streams) + (size_t)first * nc * n + t0;
+  const double* const window = a.t_window + t0;
+  auto scale_of = [&](int kernel) {  // the mixed form's table carries the power of two 2^raman_scale
+    if constexpr (sizeof(R) == 8) return density;
+    else return scalbn(density, -a.raman_scale[kernel]);
+  };
+  const bool tensor = nc == 2 && a.raman_kernels == 2;
+  const double trace_scale = scale_of(0), tensor_scale = tensor ? scale_of(1) : 0.0;
+  C* const trace = stream + ((size_t)2 * count - 1) * n;  // tensor: the last node's y row
+  const R half = R(0.5);
+  C x[V];
+  // signal 0: the trace drives of both nodes; signal 1 + q: the tensor drives of node q
+#pragma unroll 1
+  for (int signal = 0; signal <= (tensor ? count : 0); ++signal) {
+    const C* const Ex = field + (size_t)(signal - 1) * 2 * n;  // signal > 0
+    if (signal == 0) {
+#pragma unroll
+      for (int r = 0; r < V; ++r) {
+        R d[2] = {R(0), R(0)};
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          if (q < count) {
+            const C e = field[(size_t)q * nc * n + r * T];
+            d[q] = half * (e.x * e.x + e.y * e.y);
+            if (nc == 2) {
+              const C f = field[((size_t)q * 2 + 1) * n + r * T];
+              d[q] += half * (f.x * f.x + f.y * f.y);
             }
           }
         }
-        C packed;
-        packed.x = v[0];
-        packed.y = v[1];
-        B[row_slot<C>(m)] = packed;
+        x[r].x = d[0];
+        x[r].y = d[1];
       }
-      __syncthreads();
-      const C* table = spectrum_table<R>(a);
-      fft_dif_swizzled<false>(B, a.log_n_to, table, a.log_n_to + 1);
-      spectrum_product(B, kernel_spectrum<R>(a, dr == 0 ? 0 : 1), table, n, a.log_n_to);  // trace, then traceless
-      fft_dif_swizzled<true>(B, a.log_n_to, table, a.log_n_to + 1);
-    }
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-      double conv = 0.0;
-      if (drives > 0) {
-        const C z = B[row_slot<C>(bitrev(t >> 1, a.log_n_to))];
-        // irfft's 1 / (2n), with the packing's 2; the mixed form's spectrum scale taken out
-        conv = raman_scale * spectrum_unscale<R>(a, dr == 0 ? 0 : 1, (double)((t & 1) ? z.y : z.x) * inv_n);
+    } else {
+#pragma unroll
+      for (int r = 0; r < V; ++r) {
+        const C e = Ex[r * T], f = Ex[n + r * T];
+        x[r].x = half * (e.x * e.x + e.y * e.y) - half * (f.x * f.x + f.y * f.y);
+        x[r].y = e.x * f.x + e.y * f.y;
       }
-      node_sample<R>(a, Ex, Ey, Px, Py, t, conv, dr, nc, factor, self, conj);
     }
-    __syncthreads();  // the next drive's packing overwrites the row
+    Row::convolve(x, plane, stash, a.outer_twiddles, a.inner_twiddles, a.raman_table + (signal ? (size_t)2 * n : 0));
+    if (signal > 0) {
+      C* const Px = stream + (size_t)(signal - 1) * 2 * n;
+#pragma unroll
+      for (int r = 0; r < V; ++r) {
+        const C u = trace[r * T];
+        C px, py;
+        node_output<R>(a, 2, factor, window[r * T], Ex[r * T], Ex[n + r * T],
+                       trace_scale * (double)(signal == 2 ? u.y : u.x), tensor_scale * (double)x[r].x,
+                       tensor_scale * (double)x[r].y, px, py);
+        Px[r * T] = px;
+        Px[n + r * T] = py;
+      }
+    } else if (tensor) {
+#pragma unroll
+      for (int r = 0; r < V; ++r) trace[r * T] = x[r];
+    } else {
+      // rows of the stash carry the convolutions on, so that this rarer form stays a loop
+#pragma unroll
+      for (int r = 0; r < V; ++r) stash[r * T + t0] = x[r];
+#pragma unroll 1
+      for (int r = 0; r < V; ++r) {
+        const C conv = stash[r * T + t0];
+        for (int q = 0; q < count; ++q) {
+          const size_t at = (size_t)q * nc * n + r * T;
+          const C e = field[at];
+          C px, py;
+          node_output<R>(a, nc, factor, window[r * T], e, nc == 2 ? field[at + n] : e,
+                         trace_scale * (double)(q ? conv.y : conv.x), 0.0, 0.0, px, py);
+          stream[at] = px;
+          if (nc == 2) stream[at + n] = py;
+        }
+      }
+    }
   }
+}
+
+// The kernels' spectra in k_env_pairs' order: half p, register e, thread t at
+// [(2 kernel + p) n + e T + t] holds bin 2 k + p of the doubled row, k = Row::bin(t, e), over
+// 2n (the transform's normalisation) and, in the mixed form, times 2^raman_scale.
+template <class R, int LOGN>
+__global__ void __launch_bounds__(256) k_raman_table(const double2* __restrict__ spectrum, const int* scale,
+                                                     cplx<R>* __restrict__ table) {
+  using Row = regs::Row<cplx<R>, LOGN>;
+  constexpr int n = Row::N;
+  const int kernel = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int half = i >> LOGN, e = (i & (n - 1)) / Row::T, t = i % Row::T;
+  const int k = 2 * Row::bin(t, e) + half;
+  const double2* row = spectrum + (size_t)kernel * (n + 1);
+  const double2 h = k <= n ? row[k] : cconj(row[2 * n - k]);  // a real kernel's
+  const int shift = (scale ? scale[kernel] : 0) - (LOGN + 1);
+  table[(size_t)kernel * 2 * n + i] = to_c<cplx<R>>(make_double2(scalbn(h.x, shift), scalbn(h.y, shift)));
 }
 
 template <class R>
@@ -428,19 +441,82 @@ __global__ void __launch_bounds__(kNodeThreads, 1) k_env_nodes_long(EnvModalArgs
 
 }  // namespace
 
+// ---- the pairs' kernels by row length
+template <class R, int LOGN>
+constexpr size_t pairs_smem() {
+  using Row = regs::Row<cplx<R>, LOGN>;
+  return (size_t)Row::N * sizeof(cplx<R>) + Row::kPlane * sizeof(R);
+}
+// FP32 rows of 512 to 16 384 samples, FP64 rows of up to 8 192 (the row and the exchange
+// plane of the longest fill 194 KB of shared memory in either type)
+template <class R, class F>
+static cudaError_t with_row(int log_n, F&& f) {
+  switch (log_n) {
+    case 9: return f(std::integral_constant<int, 9>{});
+    case 10: return f(std::integral_constant<int, 10>{});
+    case 11: return f(std::integral_constant<int, 11>{});
+    case 12: return f(std::integral_constant<int, 12>{});
+    case 13: return f(std::integral_constant<int, 13>{});
+    case 14:
+      if constexpr (sizeof(R) == 4) return f(std::integral_constant<int, 14>{});
+      [[fallthrough]];
+    default: return cudaErrorInvalidValue;
+  }
+}
+
 cudaError_t configure_env_modal_kernels() {
   const int row = (int)(kMaxEnvelopeRowF64 * sizeof(double2));  // one FP64 row (or half a long one)
-  const void* kernels[10] = {(const void*)k_env_inverse<double>, (const void*)k_env_inverse<float>,
-                             (const void*)k_env_nodes<double>,   (const void*)k_env_nodes<float>,
-                             (const void*)k_env_forward<double>, (const void*)k_env_forward<float>,
-                             (const void*)k_env_inverse_long,    (const void*)k_env_inverse_long32,
-                             (const void*)k_env_forward_long,    (const void*)k_env_nodes_long};
-  for (int i = 0; i < 10; ++i) {
-    const int shm = row;  // an FP32 row of 16 384 samples is as long as an FP64 row of 8 192
-    cudaError_t e = cudaFuncSetAttribute(kernels[i], cudaFuncAttributeMaxDynamicSharedMemorySize, shm);
+  const void* kernels[8] = {(const void*)k_env_inverse<double>, (const void*)k_env_inverse<float>,
+                            (const void*)k_env_forward<double>, (const void*)k_env_forward<float>,
+                            (const void*)k_env_inverse_long,    (const void*)k_env_inverse_long32,
+                            (const void*)k_env_forward_long,    (const void*)k_env_nodes_long};
+  for (const void* k : kernels) {
+    // an FP32 row of 16 384 samples is as long as an FP64 row of 8 192
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, row);
+    if (e != cudaSuccess) return e;
+  }
+  auto configure = [](auto real, int log_n) {
+    using R = decltype(real);
+    return with_row<R>(log_n, [](auto log) {
+      constexpr int LOGN = decltype(log)::value;
+      return cudaFuncSetAttribute(k_env_pairs<R, LOGN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)pairs_smem<R, LOGN>());
+    });
+  };
+  for (int log_n = 9; log_n <= 14; ++log_n) {
+    cudaError_t e = configure(0.0f, log_n);
+    if (e == cudaSuccess && log_n <= 13) e = configure(0.0, log_n);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
+}
+
+void env_pair_twiddles(int n_to, const std::vector<double2>& tw, std::vector<double2>& outer,
+                       std::vector<double2>& inner) {
+  // Row's V, T, M and G (the same for either type)
+  const int log_v = n_to >= 1024 ? 5 : 4, V = 1 << log_v, T = n_to / V, M = T, G = M / V;
+  auto root = [&](long q) {  // exp(-2 pi i q / 2n), q < 2n
+    double2 w = tw[q % n_to];
+    if (q >= n_to) w = make_double2(-w.x, -w.y);
+    return w;
+  };
+  outer.resize((size_t)2 * n_to);
+  for (int p = 0; p < 2; ++p)
+    for (int f = 0; f < V; ++f)
+      for (int t = 0; t < T; ++t) outer[((size_t)p * V + f) * T + t] = root((long)(2 * f + p) * t);
+  inner.resize((size_t)V * G);
+  for (int g = 0; g < V; ++g)
+    for (int j = 0; j < G; ++j) inner[(size_t)g * G + j] = root((long)g * j * (2 * n_to / M));
+}
+
+template <class R>
+cudaError_t launch_raman_table(const EnvModalArgsT<R>& a, cplx<R>* table, cudaStream_t s) {
+  return with_row<R>(a.log_n_to, [&](auto log) {
+    constexpr int LOGN = decltype(log)::value;
+    const dim3 grid(2 * a.n_to / 256, a.n_components == 2 ? a.raman_kernels : 1);
+    k_raman_table<R, LOGN><<<grid, 256, 0, s>>>(a.raman_spectrum, sizeof(R) == 4 ? a.raman_scale : nullptr, table);
+    return cudaGetLastError();
+  });
 }
 
 template <class R>
@@ -457,13 +533,21 @@ cudaError_t launch_env_inverse(const EnvModalArgsT<R>& a, cudaStream_t s) {
 
 template <class R>
 cudaError_t launch_env_nodes(const EnvModalArgsT<R>& a, int n_nodes, cudaStream_t s) {
+  if (!a.raman_spectrum) {
+    const size_t total = (size_t)n_nodes * a.n_to;
+    k_env_kerr<R><<<(unsigned)std::min<size_t>((total + 255) / 256, 148 * 16), 256, 0, s>>>(a, n_nodes);
+    return cudaGetLastError();
+  }
   if (sizeof(R) == 8 && a.n_to > kMaxEnvelopeRowF64) {
     if constexpr (sizeof(R) == 8)
       k_env_nodes_long<<<n_nodes, kNodeThreads, (size_t)a.n_to / 2 * sizeof(double2), s>>>(a);
     return cudaGetLastError();
   }
-  k_env_nodes<R><<<n_nodes, kNodeThreads, (size_t)a.n_to * sizeof(cplx<R>), s>>>(a);
-  return cudaGetLastError();
+  return with_row<R>(a.log_n_to, [&](auto log) {
+    constexpr int LOGN = decltype(log)::value;
+    k_env_pairs<R, LOGN><<<(n_nodes + 1) / 2, regs::Row<cplx<R>, LOGN>::T, pairs_smem<R, LOGN>(), s>>>(a, n_nodes);
+    return cudaGetLastError();
+  });
 }
 
 template <class R>
@@ -481,6 +565,8 @@ template cudaError_t launch_env_inverse<double>(const EnvModalArgsT<double>&, cu
 template cudaError_t launch_env_inverse<float>(const EnvModalArgsT<float>&, cudaStream_t);
 template cudaError_t launch_env_nodes<double>(const EnvModalArgsT<double>&, int, cudaStream_t);
 template cudaError_t launch_env_nodes<float>(const EnvModalArgsT<float>&, int, cudaStream_t);
+template cudaError_t launch_raman_table<double>(const EnvModalArgsT<double>&, double2*, cudaStream_t);
+template cudaError_t launch_raman_table<float>(const EnvModalArgsT<float>&, float2*, cudaStream_t);
 template cudaError_t launch_env_forward<double>(const EnvModalArgsT<double>&, cudaStream_t);
 template cudaError_t launch_env_forward<float>(const EnvModalArgsT<float>&, cudaStream_t);
 

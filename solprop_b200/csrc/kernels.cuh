@@ -227,9 +227,8 @@ struct RamanArgs {
   // kernels formed (1: the trace; 2: trace and traceless, spectra (2, n_to + 1)); null: scalar
   const double* tensor_weights;
   int n_kernels;
-  // the mixed form's envelope products: the spectra also in complex64, each scaled by the
-  // power of two 2^scale[kernel] that brings its largest bin near one (else null)
-  float2* spectrum32;
+  // the mixed form's envelope products: the power of two 2^scale[kernel] that brings each
+  // spectrum's largest bin near one, for its FP32 table (else null)
   int* scale;
   double2* scratch;  // rows above kMaxEnvelopeRowF64: 1.5 n_to complex per kernel
 };
@@ -257,8 +256,12 @@ struct EnvModalArgsT {
   cplx<R>* spectra;               // (4, n_cols, n_omega): P, -, -, absorber
   double2* scratch;               // FP64 rows above kMaxEnvelopeRowF64: 1.5 n_to per row
   const double2* raman_spectrum;  // (raman_kernels, n_to + 1), or null without Raman
-  const float2* raman_spectrum32; // the mixed form: the spectra scaled by 2^raman_scale[k], complex64
-  const int* raman_scale;
+  const int* raman_scale;         // the mixed form: the powers of two inside raman_table
+  // the register transform of the nodes' rows (fft_regs.cuh): the spectra in its bin order,
+  // (raman_kernels, 2 n_to), its two twiddle tables
+  const cplx<R>* raman_table;
+  const cplx<R>* outer_twiddles;
+  const cplx<R>* inner_twiddles;
   int n_cols, n_omega, n_to, log_n_to, kerr, raman_mixture;
   int n_components;               // field components per node (1, or 2: rows x, y)
   int raman_kernels;              // two components: 1 (trace) or 2 (trace, traceless)
@@ -267,6 +270,12 @@ struct EnvModalArgsT {
 cudaError_t configure_env_modal_kernels();
 template <class R>
 cudaError_t launch_env_inverse(const EnvModalArgsT<R>& a, cudaStream_t s);
+// the nodes' tables: the spectra raman_spectrum (already formed) into a.raman_table's order, and
+// on the host the twiddles from exp(-2 pi i m / (2 n_to)), m < n_to
+template <class R>
+cudaError_t launch_raman_table(const EnvModalArgsT<R>& a, cplx<R>* table, cudaStream_t s);
+void env_pair_twiddles(int n_to, const std::vector<double2>& tw, std::vector<double2>& outer,
+                       std::vector<double2>& inner);
 template <class R>
 cudaError_t launch_env_nodes(const EnvModalArgsT<R>& a, int n_nodes, cudaStream_t s);
 template <class R>

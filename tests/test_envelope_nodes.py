@@ -1,0 +1,44 @@
+"""The envelope grid's node responses at every row length of the register transform, with an odd
+number of nodes (the last pair is half empty), one or two field components and one or two Raman
+kernels, against the oracle."""
+
+import dataclasses
+
+import numpy as np
+import pytest
+
+from oracle import source as S
+from solprop_b200 import _lib, grin
+from tests._cases import rel
+
+
+def _record(n_to, form):
+    rec, _ = grin.grin_record(n_to=n_to, grid=3, seed=n_to)
+    if form == "trace":
+        return dataclasses.replace(rec, raman_tensor_weights=np.array([[1.0, 0.0]]))
+    if form == "kerr":
+        return dataclasses.replace(rec, raman_enabled=False, raman_undamped=None, raman_rates=[],
+                                   raman_tensor_weights=None)
+    if form == "scalar":
+        return dataclasses.replace(
+            rec, n_modes=15, n_pol_transform=1, phi_terms=rec.phi_terms[:, ::2], prefactor_terms=rec.prefactor_terms[:, ::2],
+            synthesis=np.ascontiguousarray(rec.synthesis[::2, ::2]),
+            projection=np.ascontiguousarray(rec.projection[::2, ::2]),
+            projection_coarse=np.ascontiguousarray(rec.projection[::2, ::2]), raman_tensor_weights=None,
+            field0=rec.field0[::2])
+    return rec
+
+
+# FP64 rows differ from the oracle by the transforms' rounding, a few 1e-16 log2 n; the mixed form
+# by the FP32 transforms' and products' (the bounds of test_envelope_modal.py)
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision, bound", [("fp64", 1e-13), ("mixed", 2e-6)])
+@pytest.mark.parametrize("form", ["tensor", "trace", "scalar", "kerr"])
+@pytest.mark.parametrize("n_to", [512, 1024, 2048, 4096, 8192, 16384])
+def test_source_matches_oracle(n_to, form, precision, bound):
+    rec = _record(n_to, form)
+    rng = np.random.default_rng(n_to)
+    lab = rec.launch_field()
+    lab = (lab + 0.1 * np.exp(2j * np.pi * rng.uniform(size=(rec.n_modes, 1, 1))) * lab[:1]) * rec.active_mask
+    ws = _lib.Workspace(_lib.Problem(rec), 0, precision)
+    assert rel(ws.source(lab, 0.0), S.lab_source(rec, lab, 0.0)) < bound
