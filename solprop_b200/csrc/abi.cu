@@ -307,7 +307,7 @@ struct sp_workspace {
   bool gemm = false;
   int kpad_modes = 0, kpad_nodes = 0;
   DevBuf<double> node_field, node_streams;
-  DevBuf<uint16_t> s_parts, w_parts, modal_parts, node_parts;
+  DevBuf<uint16_t> s_parts, w_parts, modal_parts;
   DevBuf<double> proj_scratch;  // the projections' split-K partial tiles (FP32 in the mixed form)
   // the mixed-precision form's FP32 copies of the source evaluation's buffers
   int precision = SP_PRECISION_FP64;
@@ -647,7 +647,7 @@ static void eval_source_gemm(sp_workspace* ws, const double2* lab, int slot, boo
     }
     {
       KernelTimer t(ws, SP_K_PROJECT);
-      CUDA_CHECK(modal_projection_split3(ws->w_parts.p, ws->f32.node_streams.p, ws->node_parts.p,
+      CUDA_CHECK(modal_projection_split3(ws->w_parts.p, ws->f32.node_streams.p,
                                          ws->f32.proj.p, n_streams, d.n_modes, d.n_nodes, d.n_to,
                                          ws->kpad_nodes, stride, taper, status,
                                          reinterpret_cast<float*>(ws->proj_scratch.p), ws->stream));
@@ -759,7 +759,7 @@ static void eval_source_envelope_gemm(sp_workspace* ws, const double2* lab, int 
     }
     {
       KernelTimer t(ws, SP_K_PROJECT);
-      CUDA_CHECK(modal_projection_split3(ws->w_parts.p, ws->f32.node_streams.p, ws->node_parts.p, ws->f32.proj.p,
+      CUDA_CHECK(modal_projection_split3(ws->w_parts.p, ws->f32.node_streams.p, ws->f32.proj.p,
                                          1, d.n_modes, rows, n2, ws->kpad_nodes, stride, taper, status,
                                          reinterpret_cast<float*>(ws->proj_scratch.p), ws->stream));
     }
@@ -1021,7 +1021,6 @@ static void build_workspace(sp_workspace* ws) {
       ws->w_parts.upload(parts.data(), parts.size(), s);
       CUDA_CHECK(cudaStreamSynchronize(s));
       ws->modal_parts.alloc((size_t)3 * cplx_rows * d.n_to * ws->kpad_modes);
-      ws->node_parts.alloc((size_t)3 * cplx_rows * d.n_to * ws->kpad_nodes);
     } else {
       ws->node_field.alloc(field);
       ws->node_streams.alloc(3 * field);
@@ -1053,12 +1052,12 @@ static void build_workspace(sp_workspace* ws) {
   ws->norm_arrivals.zero(s);
   ws->launches = 5;
   if (ws->gemm && d.grid_kind == 1) {  // inverse, synthesis, (Raman spectrum, table,) nodes, projection, reduction,
-    ws->launches = 6 + (d.raman_enabled ? 2 : 0) + (ws->precision == SP_PRECISION_MIXED ? 2 : 0);  // forward,
-                                                                  // output; the mixed form's two split passes
+    ws->launches = 6 + (d.raman_enabled ? 2 : 0) + (ws->precision == SP_PRECISION_MIXED ? 1 : 0);  // forward,
+                                                                  // output; the mixed form's split pass
   } else if (ws->gemm) {  // inverse, synthesis, column, one projection per stream, forward, output
-    const int per_product = ws->precision == SP_PRECISION_MIXED ? 2 : 1;  // (split,) product
-    const int streams = d.plasma_enabled ? 3 : 1;  // each: (split,) product, reduction of the K splits
-    ws->launches = 4 + per_product + (per_product + 1) * streams + (d.raman_enabled ? 2 : 0);
+    const int synthesis = ws->precision == SP_PRECISION_MIXED ? 2 : 1;  // (split,) product
+    const int streams = d.plasma_enabled ? 3 : 1;  // each: product, reduction of the K splits
+    ws->launches = 4 + synthesis + 2 * streams + (d.raman_enabled ? 2 : 0);
   }
   if (ws->precision == SP_PRECISION_MIXED) build_mixed(ws, tw, rc, taps);
   if (d.grid_kind == 1 || d.raman_enabled) {  // the doubled grid's table: envelope route, Raman

@@ -299,10 +299,9 @@ cudaError_t modal_projection_f64(const double* W, const double* node_streams, do
 cudaError_t modal_synthesis_split3(const uint16_t* s_parts, const double* modal, uint16_t* modal_parts, float* E,
                                    int n_nodes, int n_modes, int n_to, int kpad, const double* taper,
                                    double* status, cudaStream_t s);
-cudaError_t modal_projection_split3(const uint16_t* w_parts, const float* node_streams, uint16_t* node_parts,
-                                    float* out, int n_streams, int n_modes, int n_nodes, int n_to, int kpad,
-                                    size_t out_stride, const double* taper, double* status, float* scratch,
-                                    cudaStream_t s);
+cudaError_t modal_projection_split3(const uint16_t* w_parts, const float* node_streams, float* out, int n_streams,
+                                    int n_modes, int n_nodes, int n_to, int kpad, size_t out_stride,
+                                    const double* taper, double* status, float* scratch, cudaStream_t s);
 cudaError_t launch_statistics(const StatisticsArgs& a, bool peaks, cudaStream_t s);
 int fft_cluster_size(int n_to);
 // a single run's transforms: one CTA per row (1) or a cluster of 2, 4 or 8 CTAs per row
