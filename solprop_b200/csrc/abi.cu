@@ -298,7 +298,7 @@ struct sp_workspace {
   DevBuf<double2> raman_spectrum;  // field-grid Raman: the damped kernel's spectrum (n_to + 1)
   DevBuf<int> raman_scale;         // the envelope products' mixed form: the spectra's powers of two
   // the envelope products' nodes: the spectra and twiddles in the register transform's order
-  DevBuf<double2> raman_table, outer_twiddles, inner_twiddles;
+  DevBuf<double2> raman_table, outer_twiddles, inner_twiddles, row_outer, row_inner;
   DevBuf<double2> env_scratch;      // the envelope products' FP64 rows above 8192 samples: 1.5 n_to per row
   DevBuf<double2> raman_scratch;    // ... and the Raman kernel's spectra
   DevBuf<ChannelTableT<double>> channels;  // a mixture's plasma channels (rate_coeff holds their tables)
@@ -316,7 +316,7 @@ struct sp_workspace {
     DevBuf<float> t_window, t_window_d, synthesis, projection, rate_coeff, taps, proj;
     DevBuf<float> node_field, node_streams;
     DevBuf<ChannelTableT<float>> channels;
-    DevBuf<float2> env_twiddles, raman_table, outer_twiddles, inner_twiddles;
+    DevBuf<float2> env_twiddles, raman_table, outer_twiddles, inner_twiddles, row_outer, row_inner;
   } f32;
   DevBuf<unsigned char> active, norm;
   DevBuf<StageScalarsDev> stage;   // kStageSlots slots
@@ -696,6 +696,9 @@ static EnvModalArgsT<R> env_modal_args(const sp_workspace* ws, const double2* la
   ea.alpha = absorber ? ws->alpha.p : nullptr;
   ea.modal_t = ws->modal_t.p;
   ea.scratch = ws->env_scratch.p;
+  ea.fine_to_coarse = ws->fine_to_coarse.p;
+  ea.row_outer = ws->row_outer.p;
+  ea.row_inner = ws->row_inner.p;
   ea.raman_spectrum = d.raman_enabled ? ws->raman_spectrum.p : nullptr;
   ea.n_cols = P.n_cols;
   ea.n_omega = d.n_omega;
@@ -711,6 +714,8 @@ static EnvModalArgsT<R> env_modal_args(const sp_workspace* ws, const double2* la
   if constexpr (sizeof(R) == 8) {
     ea.twiddles_r = ws->env_twiddles.p;
     ea.raman_table = ws->raman_table.p;
+    ea.row_outer_r = ws->row_outer.p;
+    ea.row_inner_r = ws->row_inner.p;
     ea.outer_twiddles = ws->outer_twiddles.p;
     ea.inner_twiddles = ws->inner_twiddles.p;
     ea.node_field = ws->node_field.p;
@@ -720,6 +725,8 @@ static EnvModalArgsT<R> env_modal_args(const sp_workspace* ws, const double2* la
   } else {
     ea.twiddles_r = ws->f32.env_twiddles.p;
     ea.raman_table = ws->f32.raman_table.p;
+    ea.row_outer_r = ws->f32.row_outer.p;
+    ea.row_inner_r = ws->f32.row_inner.p;
     ea.outer_twiddles = ws->f32.outer_twiddles.p;
     ea.inner_twiddles = ws->f32.inner_twiddles.p;
     ea.raman_scale = ws->raman_scale.p;
@@ -741,7 +748,12 @@ static void eval_source_envelope_gemm(sp_workspace* ws, const double2* lab, int 
   const size_t stride = (size_t)P.n_cols * n2;
   if (ws->precision == SP_PRECISION_MIXED) {
     const auto ea = env_modal_args<float>(ws, lab, slot, absorber);
-    { KernelTimer t(ws, SP_K_INVERSE); CUDA_CHECK(launch_env_inverse(ea, ws->stream)); }
+    RamanArgs ra = raman_args(ws, slot);
+    ra.scale = ws->raman_scale.p;
+    {
+      KernelTimer t(ws, SP_K_INVERSE);
+      CUDA_CHECK(launch_env_inverse(ea, d.raman_enabled ? &ra : nullptr, ws->f32.raman_table.p, ws->stream));
+    }
     {
       KernelTimer t(ws, SP_K_PROJECT);
       CUDA_CHECK(modal_synthesis_split3(ws->s_parts.p, ws->modal_t.p, ws->modal_parts.p, ws->f32.node_field.p,
@@ -749,12 +761,6 @@ static void eval_source_envelope_gemm(sp_workspace* ws, const double2* lab, int 
     }
     {
       KernelTimer t(ws, SP_K_COLUMN);
-      if (d.raman_enabled) {
-        RamanArgs ra = raman_args(ws, slot);
-        ra.scale = ws->raman_scale.p;
-        CUDA_CHECK(launch_raman_spectrum(ra, ws->stream));
-        CUDA_CHECK(launch_raman_table(ea, ws->f32.raman_table.p, ws->stream));
-      }
       CUDA_CHECK(launch_env_nodes(ea, d.n_nodes, ws->stream));
     }
     {
@@ -767,7 +773,11 @@ static void eval_source_envelope_gemm(sp_workspace* ws, const double2* lab, int 
     return;
   }
   const auto ea = env_modal_args<double>(ws, lab, slot, absorber);
-  { KernelTimer t(ws, SP_K_INVERSE); CUDA_CHECK(launch_env_inverse(ea, ws->stream)); }
+  const RamanArgs ra = raman_args(ws, slot);
+  {
+    KernelTimer t(ws, SP_K_INVERSE);
+    CUDA_CHECK(launch_env_inverse(ea, d.raman_enabled ? &ra : nullptr, ws->raman_table.p, ws->stream));
+  }
   {
     KernelTimer t(ws, SP_K_PROJECT);
     CUDA_CHECK(modal_synthesis_f64(ws->synthesis.p, ws->modal_t.p, ws->node_field.p, rows, d.n_modes, n2,
@@ -775,10 +785,6 @@ static void eval_source_envelope_gemm(sp_workspace* ws, const double2* lab, int 
   }
   {
     KernelTimer t(ws, SP_K_COLUMN);
-    if (d.raman_enabled) {
-      CUDA_CHECK(launch_raman_spectrum(raman_args(ws, slot), ws->stream));
-      if (d.n_to <= kMaxEnvelopeRowF64) CUDA_CHECK(launch_raman_table(ea, ws->raman_table.p, ws->stream));
-    }
     CUDA_CHECK(launch_env_nodes(ea, d.n_nodes, ws->stream));
   }
   {
@@ -1006,12 +1012,13 @@ static void build_workspace(sp_workspace* ws) {
   if (ws->gemm) {
     const int node_rows = d.n_nodes * d.n_pol_transform;  // two components: rows x, y per node
     const size_t field = cplx_rows * node_rows * d.n_to;
+    const size_t streams = d.grid_kind == 1 ? field : 3 * field;  // the envelope's polarisation alone
     ws->kpad_modes = modal_kpad(d.n_modes);
     ws->kpad_nodes = modal_kpad(node_rows);
     ws->proj_scratch.alloc(modal_projection_scratch(d.n_modes, node_rows, (int)cplx_rows * d.n_to));
     if (ws->precision == SP_PRECISION_MIXED) {
       ws->f32.node_field.alloc(field);
-      ws->f32.node_streams.alloc(3 * field);
+      ws->f32.node_streams.alloc(streams);
       ws->f32.node_streams.zero(s);
       std::vector<uint16_t> parts;
       split3_host(P.synthesis.data(), node_rows, d.n_modes, ws->kpad_modes, parts);
@@ -1023,7 +1030,7 @@ static void build_workspace(sp_workspace* ws) {
       ws->modal_parts.alloc((size_t)3 * cplx_rows * d.n_to * ws->kpad_modes);
     } else {
       ws->node_field.alloc(field);
-      ws->node_streams.alloc(3 * field);
+      ws->node_streams.alloc(streams);
       ws->node_streams.zero(s);
     }
   }
@@ -1051,8 +1058,9 @@ static void build_workspace(sp_workspace* ws) {
   ws->norm_arrivals.alloc(1);
   ws->norm_arrivals.zero(s);
   ws->launches = 5;
-  if (ws->gemm && d.grid_kind == 1) {  // inverse, synthesis, (Raman spectrum, table,) nodes, projection, reduction,
-    ws->launches = 6 + (d.raman_enabled ? 2 : 0) + (ws->precision == SP_PRECISION_MIXED ? 1 : 0);  // forward,
+  if (ws->gemm && d.grid_kind == 1) {  // inverse, synthesis, (long rows: Raman spectrum, table,) nodes, projection, reduction,
+    const bool long_rows = d.n_to > kMaxEnvelopeRowF64;  // the spectrum (and the mixed form's table) on their own
+    ws->launches = 6 + (d.raman_enabled && long_rows ? ws->precision == SP_PRECISION_MIXED ? 2 : 1 : 0) + (ws->precision == SP_PRECISION_MIXED ? 1 : 0);  // forward,
                                                                   // output; the mixed form's split pass
   } else if (ws->gemm) {  // inverse, synthesis, column, one projection per stream, forward, output
     const int synthesis = ws->precision == SP_PRECISION_MIXED ? 2 : 1;  // (split,) product
@@ -1077,27 +1085,44 @@ static void build_workspace(sp_workspace* ws) {
     if (!P.raman_weights.empty()) ws->raman_weights.upload(P.raman_weights.data(), P.raman_weights.size(), s);
     if (d.raman_enabled && (d.grid_kind == 0 || ws->gemm))
       ws->raman_spectrum.alloc((size_t)P.raman_kernels * (d.n_to + 1));
-    if (d.raman_enabled && d.grid_kind == 1 && ws->gemm) {
-      // the nodes' register transform (FP64 rows above kMaxEnvelopeRowF64 take the long form)
+    if (d.grid_kind == 1 && ws->gemm) {
+      // the register transform's tables, for the nodes' rows and the columns' (FP64 rows above
+      // kMaxEnvelopeRowF64 take the long form)
+      const bool mixed = ws->precision == SP_PRECISION_MIXED, rows64 = d.n_to <= kMaxEnvelopeRowF64;
+      const size_t table = d.raman_enabled ? (size_t)2 * P.raman_kernels * d.n_to : 0;
       std::vector<double2> outer, inner;
-      env_pair_twiddles(d.n_to, tw2, outer, inner);
-      const size_t table = (size_t)2 * P.raman_kernels * d.n_to;
-      if (ws->precision == SP_PRECISION_MIXED) {
-        auto narrow = [&](const std::vector<double2>& v, DevBuf<float2>& dst) {
-          std::vector<float2> f(v.size());
-          for (size_t m = 0; m < v.size(); ++m) f[m] = make_float2((float)v[m].x, (float)v[m].y);
-          dst.upload(f.data(), f.size(), s);
-          CUDA_CHECK(cudaStreamSynchronize(s));  // the host copy goes with this scope
-        };
-        narrow(outer, ws->f32.outer_twiddles);
-        narrow(inner, ws->f32.inner_twiddles);
-        ws->f32.raman_table.alloc(table);
+      auto wide = [&](const std::vector<double2>& v, DevBuf<double2>& dst) {
+        dst.upload(v.data(), v.size(), s);
+        CUDA_CHECK(cudaStreamSynchronize(s));  // the host copy is overwritten or goes with its scope
+      };
+      auto narrow = [&](const std::vector<double2>& v, DevBuf<float2>& dst) {
+        std::vector<float2> f(v.size());
+        for (size_t m = 0; m < v.size(); ++m) f[m] = make_float2((float)v[m].x, (float)v[m].y);
+        dst.upload(f.data(), f.size(), s);
+        CUDA_CHECK(cudaStreamSynchronize(s));
+      };
+      row_twiddles(d.n_to, env_column_log_v(d.n_to), tw2, outer, inner);
+      if (rows64) {
+        wide(outer, ws->row_outer);
+        wide(inner, ws->row_inner);
+      }
+      if (mixed) {
+        narrow(outer, ws->f32.row_outer);
+        narrow(inner, ws->f32.row_inner);
         ws->raman_scale.alloc(2);
-      } else if (d.n_to <= kMaxEnvelopeRowF64) {
-        ws->outer_twiddles.upload(outer.data(), outer.size(), s);
-        ws->inner_twiddles.upload(inner.data(), inner.size(), s);
-        CUDA_CHECK(cudaStreamSynchronize(s));  // the host copies go with this scope
-        ws->raman_table.alloc(table);
+      }
+      if (table) {
+        if (env_node_log_v(d.n_to) != env_column_log_v(d.n_to))
+          row_twiddles(d.n_to, env_node_log_v(d.n_to), tw2, outer, inner);
+        if (mixed) {
+          narrow(outer, ws->f32.outer_twiddles);
+          narrow(inner, ws->f32.inner_twiddles);
+          ws->f32.raman_table.alloc(table);
+        } else if (rows64) {
+          wide(outer, ws->outer_twiddles);
+          wide(inner, ws->inner_twiddles);
+          ws->raman_table.alloc(table);
+        }
       }
     }
     if (d.grid_kind == 1 && ws->gemm && d.n_to > kMaxEnvelopeRowF64) {

@@ -15,8 +15,8 @@
 //                  (k_env_kerr without Raman; k_env_nodes_long for FP64 rows of 16 384)
 //   k_env_forward  one CTA per modal column: fft of the projected row, cropped
 //
-// The columns' transforms are the shared-memory FFTs of fft.cuh over the table
-// exp(-2 pi i m / (2 n_to)), m < n_to; the nodes' the register FFT of fft_regs.cuh.  The inverse transform and the modal field are FP64
+// Every transform is the register FFT of fft_regs.cuh (FP64 rows of 16 384 samples: the halves
+// of fft_long.cuh over the table exp(-2 pi i m / (2 n_to)), m < n_to).  The inverse transform and the modal field are FP64
 // in both forms; the Kerr cubic, the Raman convolutions and the forward transform run in the
 // form's type R (FP32 in the mixed form).
 #include <algorithm>
@@ -34,31 +34,102 @@ namespace {
 constexpr double kEps0 = 8.8541878188e-12;  // vacuum permittivity (F/m), CODATA 2022, as solprop.constants
 constexpr int kEnvThreads = 1024;
 
-template <class R>
-__global__ void __launch_bounds__(kEnvThreads) k_env_inverse(EnvModalArgsT<R> a) {
-  extern __shared__ __align__(16) double2 ei_raw[];
-  const int n = a.n_to, col = blockIdx.x;
-  double2* A = ei_raw;
-  for (int k = threadIdx.x; k < n; k += blockDim.x) A[k] = make_double2(0.0, 0.0);
-  __syncthreads();
+// A column's (or kernel's) transform is one CTA's chain of passes, run once: what bounds it is
+// latency, the instructions' own fetch included, so its threads hold 16 points where the three
+// passes allow it (half the unrolled code of 32, twice the warps).  30 columns of 4 096 and two
+// Raman kernels, ncu: the inverse and the kernels' spectra 32.6 + 28.6 us with shared-memory
+// radix-4 transforms in launches of their own -> 32.4 us, the FP32 forward 14.7 -> 13.4 (with
+// 32 points per thread 28.6); FP64 columns of 8 192: 66 + 46 -> 57 us, the forward 34 us.
+constexpr int column_log_v(int log_n) { return log_n <= 12 ? 4 : 5; }
+template <class C, int LOGN>
+using ColumnRow = regs::Row<C, LOGN, column_log_v(LOGN)>;
+
+// The Raman kernels' spectra in k_env_pairs' order (rows of up to 8 192; longer ones take
+// k_raman_kernel and k_raman_table): one CTA per kernel and half p transforms the damped
+// kernel's samples s and s + n together, K[s] + K[s + n] for the even bins of the doubled row
+// and (K[s] - K[s + n]) w_2n^s for the odd ones.  Both halves scale by the power of two that
+// brings the kernel's sum of magnitudes, a bound of its bins, into [1, 2) (the mixed form).
+template <class R, int LOGN>
+__device__ __forceinline__ void raman_row(const EnvModalArgsT<R>& a, const RamanArgs& ra, cplx<R>* table, int kernel,
+                                          int half, double* plane) {
+  using Row = ColumnRow<double2, LOGN>;
+  constexpr int n = Row::N, T = Row::T, V = Row::V;
+  const int t0 = threadIdx.x;
+  double2 x[V];
+  double sum = 0.0;
+#pragma unroll 4
+  for (int r = 0; r < V; ++r) {
+    const double k0 = raman_sample(ra, kernel, t0 + r * T), k1 = raman_sample(ra, kernel, n + t0 + r * T);
+    sum += fabs(k0) + fabs(k1);
+    plane[r * T + t0] = half ? k0 - k1 : k0 + k1;  // each thread its own places
+  }
+#pragma unroll
+  for (int r = 0; r < V; ++r) {
+    x[r] = make_double2(plane[r * T + t0], 0.0);
+    if (half) x[r] = regs::rotate64<false>(x[r], r * (32 / V));
+  }
+  int shift = 0;
+  if (sizeof(R) == 4) {
+    __shared__ double part[T / 32];
+    for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+    if (t0 % 32 == 0) part[t0 / 32] = sum;
+    __syncthreads();
+    double all = 0.0;
+    for (int w = 0; w < T / 32; ++w) all += part[w];
+    all *= ra.dt;
+    if (all > 0.0) shift = -ilogb(all);
+    if (t0 == 0 && half == 0) ra.scale[kernel] = shift;
+  }
+  Row::forward(x, plane, a.row_outer, a.row_inner, half);
+  const double f = scalbn(ra.dt, shift - (LOGN + 1));  // the convolution's 1 / 2n inside
+  cplx<R>* out = table + ((size_t)kernel * 2 + half) * n;
+#pragma unroll
+  for (int e = 0; e < V; ++e)
+    out[regs::Row<cplx<R>, LOGN>::place(Row::bin(t0, e))] = to_c<cplx<R>>(cscale(f, x[e]));
+}
+
+// The inverse transform of a column: the padded spectrum is gathered in the register
+// transform's bin order (fine_to_coarse: -1 where the band is cropped), so that the inverse
+// passes leave a(t) in natural order; the in-stage absorber's -alpha a / 2 goes forward from
+// there and its bins are scattered to the cropped spectrum (stage output masks it).
+// The Raman kernels' spectra take their CTAs of the same launch, ahead of the columns': they
+// are as long a chain, and nothing of them depends on the field.
+template <class R, int LOGN>
+__global__ void __launch_bounds__(ColumnRow<double2, LOGN>::T)
+    k_env_inverse(EnvModalArgsT<R> a, RamanArgs ra, cplx<R>* table, int raman_rows) {
+  using Row = ColumnRow<double2, LOGN>;
+  constexpr int n = Row::N, T = Row::T, V = Row::V;
+  extern __shared__ __align__(16) double ei_plane[];
+  if ((int)blockIdx.x < raman_rows) {
+    raman_row<R, LOGN>(a, ra, table, blockIdx.x / 2, blockIdx.x % 2, ei_plane);
+    return;
+  }
+  const int col = blockIdx.x - raman_rows, t0 = threadIdx.x;
   const double2* lab = a.lab + (size_t)col * a.n_omega;
-  for (int j = threadIdx.x; j < a.n_omega; j += blockDim.x) A[a.crop[j]] = lab[j];
-  __syncthreads();
-  fft_dif_inplace(A, a.log_n_to, a.twiddles, a.log_n_to + 1, /*inverse=*/true);
+  double2 x[V];
+#pragma unroll
+  for (int e = 0; e < V; ++e) {
+    const int j = a.fine_to_coarse[Row::bin(t0, e)];
+    x[e] = j >= 0 ? lab[j] : make_double2(0.0, 0.0);
+  }
+  Row::inverse(x, ei_plane, a.row_outer, a.row_inner, 0);
   const double inv_n = 1.0 / (double)n;  // scipy's ifft carries 1 / n_to
-  double2* row = reinterpret_cast<double2*>(a.modal_t + (size_t)col * 2 * n);
-  for (int t = threadIdx.x; t < n; t += blockDim.x) row[t] = cscale(inv_n, A[bitrev(t, a.log_n_to)]);
+  double2* row = reinterpret_cast<double2*>(a.modal_t + (size_t)col * 2 * n) + t0;
+#pragma unroll
+  for (int r = 0; r < V; ++r) {
+    x[r] = cscale(inv_n, x[r]);
+    row[r * T] = x[r];
+  }
   if (!a.alpha) return;
-  // the in-stage absorber -alpha a / 2, transformed and cropped (stage output masks it); the
-  // row of shared memory is reused, a(t) read back from the modal field just written
-  __syncthreads();
-  double2* B = A;
-  for (int t = threadIdx.x; t < n; t += blockDim.x) B[t] = cscale(-0.5 * a.alpha[t], row[t]);
-  __syncthreads();
-  fft_dif_inplace(B, a.log_n_to, a.twiddles, a.log_n_to + 1, /*inverse=*/false);
+#pragma unroll
+  for (int r = 0; r < V; ++r) x[r] = cscale(-0.5 * a.alpha[t0 + r * T], x[r]);
+  Row::forward(x, ei_plane, a.row_outer, a.row_inner, 0);
   cplx<R>* absorber = a.spectra + (size_t)3 * a.n_cols * a.n_omega + (size_t)col * a.n_omega;
-  for (int j = threadIdx.x; j < a.n_omega; j += blockDim.x)
-    absorber[j] = to_c<cplx<R>>(B[bitrev((int)a.crop[j], a.log_n_to)]);
+#pragma unroll
+  for (int e = 0; e < V; ++e) {
+    const int j = a.fine_to_coarse[Row::bin(t0, e)];
+    if (j >= 0) absorber[j] = to_c<cplx<R>>(x[e]);
+  }
 }
 
 constexpr int kNodeThreads = 512;
@@ -276,18 +347,24 @@ __global__ void __launch_bounds__(256) k_raman_table(const double2* __restrict__
   table[(size_t)kernel * 2 * n + i] = to_c<cplx<R>>(make_double2(scalbn(h.x, shift), scalbn(h.y, shift)));
 }
 
-template <class R>
-__global__ void __launch_bounds__(kEnvThreads) k_env_forward(EnvModalArgsT<R> a) {
+// The forward transform of a projected column, its bins scattered to the cropped spectrum
+template <class R, int LOGN>
+__global__ void __launch_bounds__(ColumnRow<cplx<R>, LOGN>::T) k_env_forward(EnvModalArgsT<R> a) {
   using C = cplx<R>;
+  using Row = ColumnRow<C, LOGN>;
   extern __shared__ __align__(16) unsigned char ef_raw[];
-  const int n = a.n_to, col = blockIdx.x;
-  C* A = reinterpret_cast<C*>(ef_raw);
-  const C* row = reinterpret_cast<const C*>(a.projected) + (size_t)col * n;
-  for (int t = threadIdx.x; t < n; t += blockDim.x) A[t] = row[t];
-  __syncthreads();
-  fft_dif_inplace(A, a.log_n_to, a.twiddles_r, a.log_n_to + 1, /*inverse=*/false);
+  const int col = blockIdx.x, t0 = threadIdx.x;
+  const C* row = reinterpret_cast<const C*>(a.projected) + (size_t)col * Row::N + t0;
+  C x[Row::V];
+#pragma unroll
+  for (int r = 0; r < Row::V; ++r) x[r] = row[r * Row::T];
+  Row::forward(x, reinterpret_cast<R*>(ef_raw), a.row_outer_r, a.row_inner_r, 0);
   C* spectra = a.spectra + (size_t)col * a.n_omega;
-  for (int j = threadIdx.x; j < a.n_omega; j += blockDim.x) spectra[j] = A[bitrev((int)a.crop[j], a.log_n_to)];
+#pragma unroll
+  for (int e = 0; e < Row::V; ++e) {
+    const int j = a.fine_to_coarse[Row::bin(t0, e)];
+    if (j >= 0) spectra[j] = x[e];
+  }
 }
 
 // ---- FP64 rows of 16 384 samples: the halves of fft_long.cuh over each row's scratch
@@ -464,14 +541,13 @@ static cudaError_t with_row(int log_n, F&& f) {
   }
 }
 
+template <class C, int LOGN>
+constexpr size_t plane_smem() { return ColumnRow<C, LOGN>::kPlane * sizeof(typename ColumnRow<C, LOGN>::R); }
+
 cudaError_t configure_env_modal_kernels() {
-  const int row = (int)(kMaxEnvelopeRowF64 * sizeof(double2));  // one FP64 row (or half a long one)
-  const void* kernels[8] = {(const void*)k_env_inverse<double>, (const void*)k_env_inverse<float>,
-                            (const void*)k_env_forward<double>, (const void*)k_env_forward<float>,
-                            (const void*)k_env_inverse_long,    (const void*)k_env_inverse_long32,
-                            (const void*)k_env_forward_long,    (const void*)k_env_nodes_long};
-  for (const void* k : kernels) {
-    // an FP32 row of 16 384 samples is as long as an FP64 row of 8 192
+  const int row = (int)(kMaxEnvelopeRowF64 * sizeof(double2));  // half a long FP64 row
+  for (const void* k : {(const void*)k_env_inverse_long, (const void*)k_env_inverse_long32,
+                        (const void*)k_env_forward_long, (const void*)k_env_nodes_long}) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, row);
     if (e != cudaSuccess) return e;
   }
@@ -479,8 +555,15 @@ cudaError_t configure_env_modal_kernels() {
     using R = decltype(real);
     return with_row<R>(log_n, [](auto log) {
       constexpr int LOGN = decltype(log)::value;
-      return cudaFuncSetAttribute(k_env_pairs<R, LOGN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)pairs_smem<R, LOGN>());
+      const auto limit = cudaFuncAttributeMaxDynamicSharedMemorySize;
+      cudaError_t e = cudaFuncSetAttribute(k_env_pairs<R, LOGN>, limit, (int)pairs_smem<R, LOGN>());
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_env_forward<R, LOGN>, limit, (int)plane_smem<cplx<R>, LOGN>());
+      if constexpr (LOGN <= 13) {
+        if (e == cudaSuccess)
+          e = cudaFuncSetAttribute(k_env_inverse<R, LOGN>, limit, (int)plane_smem<double2, LOGN>());
+      }
+      return e;
     });
   };
   for (int log_n = 9; log_n <= 14; ++log_n) {
@@ -491,12 +574,15 @@ cudaError_t configure_env_modal_kernels() {
   return cudaSuccess;
 }
 
-void env_pair_twiddles(int n_to, const std::vector<double2>& tw, std::vector<double2>& outer,
-                       std::vector<double2>& inner) {
+int env_column_log_v(int n_to) { return column_log_v(31 - __builtin_clz((unsigned)n_to)); }
+int env_node_log_v(int n_to) { return regs::default_log_v(31 - __builtin_clz((unsigned)n_to)); }
+
+void row_twiddles(int n_to, int log_v, const std::vector<double2>& tw, std::vector<double2>& outer,
+                  std::vector<double2>& inner) {
   // Row's V, T, M and G (the same for either type)
-  const int log_v = n_to >= 1024 ? 5 : 4, V = 1 << log_v, T = n_to / V, M = T, G = M / V;
+  const int V = 1 << log_v, T = n_to / V, M = T, G = M / V;
   auto root = [&](long q) {  // exp(-2 pi i q / 2n), q < 2n
-    double2 w = tw[q % n_to];
+    double2 w = tw[q & (n_to - 1)];
     if (q >= n_to) w = make_double2(-w.x, -w.y);
     return w;
   };
@@ -510,25 +596,29 @@ void env_pair_twiddles(int n_to, const std::vector<double2>& tw, std::vector<dou
 }
 
 template <class R>
-cudaError_t launch_raman_table(const EnvModalArgsT<R>& a, cplx<R>* table, cudaStream_t s) {
-  return with_row<R>(a.log_n_to, [&](auto log) {
-    constexpr int LOGN = decltype(log)::value;
-    const dim3 grid(2 * a.n_to / 256, a.n_components == 2 ? a.raman_kernels : 1);
-    k_raman_table<R, LOGN><<<grid, 256, 0, s>>>(a.raman_spectrum, sizeof(R) == 4 ? a.raman_scale : nullptr, table);
-    return cudaGetLastError();
-  });
-}
-
-template <class R>
-cudaError_t launch_env_inverse(const EnvModalArgsT<R>& a, cudaStream_t s) {
+cudaError_t launch_env_inverse(const EnvModalArgsT<R>& a, const RamanArgs* raman, cplx<R>* table, cudaStream_t s) {
+  const int kernels = !raman ? 0 : a.n_components == 2 ? a.raman_kernels : 1;
   if (a.n_to > kMaxEnvelopeRowF64) {
     const size_t half = (size_t)a.n_to / 2 * sizeof(double2);
     if constexpr (sizeof(R) == 8) k_env_inverse_long<<<a.n_cols, kEnvThreads, half, s>>>(a);
     else k_env_inverse_long32<<<a.n_cols, kEnvThreads, half, s>>>(a);
-    return cudaGetLastError();
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess || !raman) return e;
+    e = launch_raman_spectrum(*raman, s);
+    if (e != cudaSuccess || sizeof(R) == 8) return e;  // k_env_nodes_long reads the spectrum itself
+    return with_row<R>(a.log_n_to, [&](auto log) {
+      k_raman_table<R, decltype(log)::value><<<dim3(2 * a.n_to / 256, kernels), 256, 0, s>>>(a.raman_spectrum,
+                                                                                           raman->scale, table);
+      return cudaGetLastError();
+    });
   }
-  k_env_inverse<R><<<a.n_cols, kEnvThreads, (size_t)a.n_to * sizeof(double2), s>>>(a);
-  return cudaGetLastError();
+  return with_row<R>(a.log_n_to, [&](auto log) {
+    constexpr int LOGN = decltype(log)::value;
+    if constexpr (LOGN <= 13)
+      k_env_inverse<R, LOGN><<<a.n_cols + 2 * kernels, ColumnRow<double2, LOGN>::T, plane_smem<double2, LOGN>(), s>>>(
+          a, raman ? *raman : RamanArgs{}, table, 2 * kernels);
+    return cudaGetLastError();
+  });
 }
 
 template <class R>
@@ -557,16 +647,17 @@ cudaError_t launch_env_forward(const EnvModalArgsT<R>& a, cudaStream_t s) {
       k_env_forward_long<<<a.n_cols, kEnvThreads, (size_t)a.n_to / 2 * sizeof(double2), s>>>(a);
     return cudaGetLastError();
   }
-  k_env_forward<R><<<a.n_cols, kEnvThreads, (size_t)a.n_to * sizeof(cplx<R>), s>>>(a);
-  return cudaGetLastError();
+  return with_row<R>(a.log_n_to, [&](auto log) {
+    constexpr int LOGN = decltype(log)::value;
+    k_env_forward<R, LOGN><<<a.n_cols, ColumnRow<cplx<R>, LOGN>::T, plane_smem<cplx<R>, LOGN>(), s>>>(a);
+    return cudaGetLastError();
+  });
 }
 
-template cudaError_t launch_env_inverse<double>(const EnvModalArgsT<double>&, cudaStream_t);
-template cudaError_t launch_env_inverse<float>(const EnvModalArgsT<float>&, cudaStream_t);
+template cudaError_t launch_env_inverse<double>(const EnvModalArgsT<double>&, const RamanArgs*, double2*, cudaStream_t);
+template cudaError_t launch_env_inverse<float>(const EnvModalArgsT<float>&, const RamanArgs*, float2*, cudaStream_t);
 template cudaError_t launch_env_nodes<double>(const EnvModalArgsT<double>&, int, cudaStream_t);
 template cudaError_t launch_env_nodes<float>(const EnvModalArgsT<float>&, int, cudaStream_t);
-template cudaError_t launch_raman_table<double>(const EnvModalArgsT<double>&, double2*, cudaStream_t);
-template cudaError_t launch_raman_table<float>(const EnvModalArgsT<float>&, float2*, cudaStream_t);
 template cudaError_t launch_env_forward<double>(const EnvModalArgsT<double>&, cudaStream_t);
 template cudaError_t launch_env_forward<float>(const EnvModalArgsT<float>&, cudaStream_t);
 

@@ -1,5 +1,5 @@
-// A complex FFT of N = 2^LOGN points held in the registers of one CTA, for the convolutions
-// of the envelope grid's nodes: N / V threads of V points each (V = 32; 16 at N = 512).
+// A complex FFT of N = 2^LOGN points held in the registers of one CTA, for the envelope
+// grid: N / V threads of V points each (V = 32, or 16 for short rows).
 //
 // The factorisation is N = V x V x G, G = N / V^2 <= 16, decimation in frequency:
 //   pass 1  thread t holds x[t + r T], r < V (T = N / V threads): a V-point DFT over r, the
@@ -101,10 +101,12 @@ __device__ __forceinline__ void dft_dit_inverse(C* x) {
 // may keep in registers from the forward transform to the inverse, which reads the same
 // twiddles, and the row is spilled to make room for them.
 
-template <class C, int LOGN>
+constexpr int default_log_v(int log_n) { return log_n >= 10 ? 5 : 4; }
+
+template <class C, int LOGN, int LOGV = default_log_v(LOGN)>
 struct Row {
   using R = decltype(C{}.x);
-  static constexpr int kLogV = LOGN >= 10 ? 5 : 4, V = 1 << kLogV;
+  static constexpr int kLogV = LOGV, V = 1 << kLogV;
   static constexpr int N = 1 << LOGN, T = N / V, M = T, G = M / V;
   static constexpr int kLogG = LOGN - 2 * kLogV;
   static_assert(kLogG >= 0 && G <= V && G <= 32 && T >= 32, "N = V V G with G threads of a warp per row");
@@ -169,6 +171,13 @@ struct Row {
   static __host__ __device__ constexpr int bin(int t, int e) {
     if constexpr (G == 1) return t + V * rev(e, kLogV);
     else return t / G + V * ((t % G) * (V / G) + e / G + V * rev(e % G, kLogG));
+  }
+
+  // where bin k of a half lies among the points: register e of thread t at e T + t
+  static __device__ __forceinline__ int place(int k) {
+    const int f = k % V, g = (k / V) % V, h = k / (V * V);
+    if constexpr (G == 1) return rev(g, kLogV) * T + f;
+    else return ((g % (V / G)) * G + rev(h, kLogG)) * T + f * G + g / (V / G);
   }
 
   // the inverse (unnormalised) of forward: points of pass 3 -> natural x[t + r T]

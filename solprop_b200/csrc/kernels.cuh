@@ -232,6 +232,23 @@ struct RamanArgs {
   int* scale;
   double2* scratch;  // rows above kMaxEnvelopeRowF64: 1.5 n_to complex per kernel
 };
+// sample s < 2 n_to of a damped kernel.  One component: f_R sum_r u_r(s) e^(-g_r s dt); a mixture
+// (passes/responses.py:293-334): sum_c rho_c f_c sum_r u_r(s) e^(-g_r s dt), rows in component order
+__device__ __forceinline__ double raman_sample(const RamanArgs& a, int kernel, int s) {
+  const StageScalarsDev& st = *a.stage;
+  const double* weights = a.tensor_weights;  // (rows, 2), or null for one component
+  const double delay = (double)s * a.dt;
+  double total = 0.0;
+  for (int c = 0; c < a.n_components; ++c) {
+    double k = 0.0;
+    for (int r = a.first_row[c]; r < a.first_row[c + 1]; ++r) {
+      const double damped = a.undamped[(size_t)r * 2 * a.n_to + s] * exp(-st.raman_rates[r] * delay);
+      k += weights ? weights[2 * r + kernel] * damped : damped;
+    }
+    total += a.n_components > 1 ? st.raman_densities[c] * a.fraction[c] * k : a.fraction[c] * k;
+  }
+  return total;
+}
 cudaError_t configure_raman_kernels();
 cudaError_t launch_raman_spectrum(const RamanArgs& a, cudaStream_t s);  // the kernel's spectrum alone
 
@@ -262,20 +279,27 @@ struct EnvModalArgsT {
   const cplx<R>* raman_table;
   const cplx<R>* outer_twiddles;
   const cplx<R>* inner_twiddles;
+  const double2* row_outer;       // the columns' transforms (rows of up to kMaxEnvelopeRowF64), FP64
+  const double2* row_inner;
+  const cplx<R>* row_outer_r;     // ... and in the form's type
+  const cplx<R>* row_inner_r;
+  const int* fine_to_coarse;      // (n_to): the coarse bin of a fine one, or -1
   int n_cols, n_omega, n_to, log_n_to, kerr, raman_mixture;
   int n_components;               // field components per node (1, or 2: rows x, y)
   int raman_kernels;              // two components: 1 (trace) or 2 (trace, traceless)
   double kerr_coefficient, kerr_self, kerr_conjugate;
 };
 cudaError_t configure_env_modal_kernels();
+// with raman (its scale set in the mixed form), also the Raman kernels' spectra into table, the
+// nodes' a.raman_table
 template <class R>
-cudaError_t launch_env_inverse(const EnvModalArgsT<R>& a, cudaStream_t s);
-// the nodes' tables: the spectra raman_spectrum (already formed) into a.raman_table's order, and
-// on the host the twiddles from exp(-2 pi i m / (2 n_to)), m < n_to
-template <class R>
-cudaError_t launch_raman_table(const EnvModalArgsT<R>& a, cplx<R>* table, cudaStream_t s);
-void env_pair_twiddles(int n_to, const std::vector<double2>& tw, std::vector<double2>& outer,
-                       std::vector<double2>& inner);
+cudaError_t launch_env_inverse(const EnvModalArgsT<R>& a, const RamanArgs* raman, cplx<R>* table, cudaStream_t s);
+int env_column_log_v(int n_to);  // log2 of the points per thread of the columns' and the nodes' rows
+int env_node_log_v(int n_to);
+// the register transform's tables for V = 2^log_v points per thread, from exp(-2 pi i m / (2 n_to)),
+// m < n_to (fft_regs.cuh)
+void row_twiddles(int n_to, int log_v, const std::vector<double2>& tw, std::vector<double2>& outer,
+                  std::vector<double2>& inner);
 template <class R>
 cudaError_t launch_env_nodes(const EnvModalArgsT<R>& a, int n_nodes, cudaStream_t s);
 template <class R>

@@ -43,28 +43,8 @@ __global__ void __launch_bounds__(kRamanThreads) k_raman_kernel(RamanArgs a) {
   extern __shared__ __align__(16) double2 rk_raw[];
   const int n = a.n_to, kernel = blockIdx.x;
   double2* B = rk_raw;
-  const StageScalarsDev& st = *a.stage;
-  const double* weights = a.tensor_weights;  // (rows, 2), or null for one component
-  // one component: f_R sum_r u_r(s) e^(-g_r s dt); a mixture (passes/responses.py:293-334):
-  // sum_c rho_c f_c sum_r u_r(s) e^(-g_r s dt), rows in component order
-  const bool mixture = a.n_components > 1;
   auto packed = [&](int m) {
-    double v[2];
-    for (int q = 0; q < 2; ++q) {
-      const int s = 2 * m + q;
-      const double delay = (double)s * a.dt;
-      double total = 0.0;
-      for (int c = 0; c < a.n_components; ++c) {
-        double k = 0.0;
-        for (int r = a.first_row[c]; r < a.first_row[c + 1]; ++r) {
-          const double damped = a.undamped[(size_t)r * 2 * n + s] * exp(-st.raman_rates[r] * delay);
-          k += weights ? weights[2 * r + kernel] * damped : damped;
-        }
-        total += mixture ? st.raman_densities[c] * a.fraction[c] * k : a.fraction[c] * k;
-      }
-      v[q] = total;
-    }
-    return make_double2(v[0], v[1]);
+    return make_double2(raman_sample(a, kernel, 2 * m), raman_sample(a, kernel, 2 * m + 1));
   };
   double2* spectrum = a.spectrum + (size_t)kernel * (n + 1);
   double largest = 0.0;
