@@ -44,11 +44,12 @@ def test_source_matches_oracle(n_to, form, precision, bound):
     assert rel(ws.source(lab, 0.0), S.lab_source(rec, lab, 0.0)) < bound
 
 
-# the mixed form's products: mode counts about the projection's 32- and 64-wide tiles and the
-# synthesis's 64-wide K slices, rows of nodes that fill neither a 128-row tile nor a K slice
+# the products: mode counts about the projections' 32- and 64-wide tiles and the synthesis's 16-
+# and 64-wide K slices, rows of nodes that fill neither a tile nor a K slice
 @pytest.mark.gpu
+@pytest.mark.parametrize("precision, bound", [("fp64", 1e-13), ("mixed", 2e-6)])
 @pytest.mark.parametrize("modes", [2, 32, 33, 64, 65, 130])
-def test_products_at_mode_counts(modes):
+def test_products_at_mode_counts(modes, precision, bound):
     rec, _ = grin.grin_record(n_to=512, grid=13, seed=modes)
     idx = np.arange(modes) % rec.n_modes
     weight = np.random.default_rng(modes).uniform(0.5, 1.0, modes) * np.sqrt(30 / max(modes, 30))
@@ -58,5 +59,5 @@ def test_products_at_mode_counts(modes):
         projection=np.ascontiguousarray(rec.projection[idx] * weight[:, None]),
         projection_coarse=np.ascontiguousarray(rec.projection[idx] * weight[:, None]), field0=rec.field0[idx])
     lab = rec.launch_field()
-    ws = _lib.Workspace(_lib.Problem(rec), 0, "mixed")
-    assert rel(ws.source(lab, 0.0), S.lab_source(rec, lab, 0.0)) < 2e-6
+    ws = _lib.Workspace(_lib.Problem(rec), 0, precision)
+    assert rel(ws.source(lab, 0.0), S.lab_source(rec, lab, 0.0)) < bound
