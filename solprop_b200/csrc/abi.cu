@@ -816,8 +816,9 @@ static void eval_source(sp_workspace* ws, const double2* lab, int slot, const do
     EnvelopeArgs ea{};
     ea.stage = ws->stage.p + slot;
     ea.lab = lab;
-    ea.crop = ws->crop.p;
-    ea.twiddles = ws->env_twiddles.p;
+    ea.fine_to_coarse = ws->fine_to_coarse.p;
+    ea.outer = ws->row_outer.p;
+    ea.inner = ws->row_inner.p;
     ea.t_window = ws->t_window.p;
     ea.raman_undamped = d.raman_enabled ? ws->raman_undamped.p : nullptr;
     ea.spectra = ws->spectra.p;
@@ -1085,11 +1086,11 @@ static void build_workspace(sp_workspace* ws) {
     if (!P.raman_weights.empty()) ws->raman_weights.upload(P.raman_weights.data(), P.raman_weights.size(), s);
     if (d.raman_enabled && (d.grid_kind == 0 || ws->gemm))
       ws->raman_spectrum.alloc((size_t)P.raman_kernels * (d.n_to + 1));
-    if (d.grid_kind == 1 && ws->gemm) {
+    if (d.grid_kind == 1) {
       // the register transform's tables, for the nodes' rows and the columns' (FP64 rows above
       // kMaxEnvelopeRowF64 take the long form)
       const bool mixed = ws->precision == SP_PRECISION_MIXED, rows64 = d.n_to <= kMaxEnvelopeRowF64;
-      const size_t table = d.raman_enabled ? (size_t)2 * P.raman_kernels * d.n_to : 0;
+      const size_t table = d.raman_enabled && ws->gemm ? (size_t)2 * P.raman_kernels * d.n_to : 0;
       std::vector<double2> outer, inner;
       auto wide = [&](const std::vector<double2>& v, DevBuf<double2>& dst) {
         dst.upload(v.data(), v.size(), s);

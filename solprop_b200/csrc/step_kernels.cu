@@ -553,12 +553,22 @@ __global__ void __launch_bounds__(256) k_rk_stage_input(RkArgs a, RkCoeffs c) {
   const StageScalarsDev& st = *a.stage;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
     const double2 x = combine_terms(st.phi_w, st.n_phi, a.phi_terms, a.n, i);
-    double2 comb = make_double2(0.0, 0.0);
-    for (int j = 0; j < c.stage; ++j) comb = cadd(comb, cscale(c.a[j], a.stages[(size_t)j * a.n + i]));
+    // every row's load before the first sum: the stages' count is known only at run time
     const double2 y = a.state[i];
+    double2 k[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j)
+      if (j < c.stage) k[j] = a.stages[(size_t)j * a.n + i];
+    double2 comb = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int j = 0; j < 6; ++j)
+      if (j < c.stage) comb = cadd(comb, cscale(c.a[j], k[j]));
     const double2 inner = cadd(y, cscale(c.dz, comb));
-    a.lab[i] = cmul(cexp(x), inner);
-    a.back[i] = cexp(make_double2(-x.x, -x.y));
+    double sn, cs;
+    sincos(x.y, &sn, &cs);
+    const double grow = exp(x.x), decay = exp(-x.x);
+    a.lab[i] = cmul(make_double2(grow * cs, grow * sn), inner);
+    a.back[i] = make_double2(decay * cs, -(decay * sn));
   }
 }
 

@@ -61,3 +61,19 @@ def test_products_at_mode_counts(modes, precision, bound):
     lab = rec.launch_field()
     ws = _lib.Workspace(_lib.Problem(rec), 0, precision)
     assert rel(ws.source(lab, 0.0), S.lab_source(rec, lab, 0.0)) < bound
+
+
+# one mode on one node: the cluster kernel's row lengths, with and without the Raman halves
+@pytest.mark.gpu
+@pytest.mark.parametrize("raman", [True, False])
+@pytest.mark.parametrize("n_to", [512, 1024, 2048, 4096])
+def test_single_mode_source(n_to, raman):
+    rec = _record(n_to, "scalar" if raman else "kerr")
+    rec = dataclasses.replace(
+        rec, n_modes=1, n_nodes=1, n_pol_transform=1, phi_terms=rec.phi_terms[:, :1],
+        prefactor_terms=rec.prefactor_terms[:, :1], synthesis=np.array([[3e6]]), projection=np.array([[1 / 3e6]]),
+        projection_coarse=np.array([[1 / 3e6]]), absorber_scheme="none", temporal_absorber_fine=None,
+        field0=rec.field0[:1])
+    lab = rec.launch_field()
+    ws = _lib.Workspace(_lib.Problem(rec), 0)
+    assert rel(ws.source(lab, 0.0), S.lab_source(rec, lab, 0.0)) < 1e-13
