@@ -447,6 +447,21 @@ sp_status sp_mlp_mse(const float* Y, const float* T, int M, int N, float* dY, fl
 /* One Adam step (bias-corrected, step >= 1) on n FP32 weights. */
 sp_status sp_mlp_adam(float* w, const float* grad, float* m1, float* m2, size_t n, float lr,
                       float beta1, float beta2, float eps, int step, void* stream);
+/* One training layer's backward pass up to its products: dz = dA gelu'(pre) (pre NULL: dA), its
+ * BF16 copy dz16 (M, N) and transpose dz16t (N, rows_pad), either NULL, and the bias gradient db.
+ * sp_mlp_first_layer_backward: the first layer's gradients, x (M, K) with K <= 8. */
+sp_status sp_mlp_layer_backward(const float* dA, const float* pre, int M, int N, void* dz16, void* dz16t,
+                                int rows_pad, float* db, void* stream);
+sp_status sp_mlp_first_layer_backward(const float* dA, const float* pre, const float* x, int ldx, int M,
+                                      int N, int K, float* dW, float* db, void* stream);
+/* sp_mlp_adam for up to 16 parameters, sp_mlp_to_bf16 / sp_mlp_transpose_bf16 for up to 8 matrices, in
+ * one launch: copy[q] (rows, cols_out) and transpose[q] (cols, rows_pad), either NULL. */
+sp_status sp_mlp_adam_batch(int count, float* const* w, const float* const* grad, float* const* m1,
+                            float* const* m2, const size_t* n, float lr, float beta1, float beta2,
+                            float eps, int step, void* stream);
+sp_status sp_mlp_convert_batch(int count, int src_bf16, const void* const* src, const int* rows,
+                               const int* cols, const int* ld, void* const* copy, const int* cols_out,
+                               void* const* transpose, const int* rows_pad, void* stream);
 /* Ensemble statistics of Y (members, M, N) of log10 spectral densities: mean (M, N) and,
  * per row, the disagreement: the standard deviation over members of each output weighted
  * by 10^mean (the mean spectrum's energy there), over the summed weights. */

@@ -176,6 +176,16 @@ SIGNATURES = {
                              C.c_void_p, C.c_void_p]),
     "sp_mlp_adam": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_float,
                               C.c_float, C.c_float, C.c_float, C.c_int, C.c_void_p]),
+    "sp_mlp_layer_backward": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_void_p,
+                                        C.c_int, C.c_void_p, C.c_void_p]),
+    "sp_mlp_first_layer_backward": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int,
+                                              C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]),
+    "sp_mlp_adam_batch": (C.c_int, [C.c_int, C.POINTER(C.c_void_p), C.POINTER(C.c_void_p), C.POINTER(C.c_void_p),
+                                    C.POINTER(C.c_void_p), C.POINTER(C.c_size_t), C.c_float, C.c_float, C.c_float,
+                                    C.c_float, C.c_int, C.c_void_p]),
+    "sp_mlp_convert_batch": (C.c_int, [C.c_int, C.c_int, C.POINTER(C.c_void_p), C.POINTER(C.c_int),
+                                       C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_void_p),
+                                       C.POINTER(C.c_int), C.POINTER(C.c_void_p), C.POINTER(C.c_int), C.c_void_p]),
     "sp_mlp_ensemble_stats": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p,
                                         C.c_void_p]),
     "sp_workspace_destroy": (C.c_int, [C.c_void_p]),

@@ -170,6 +170,97 @@ __global__ void k_bias_grad(const float* dZ, int M, int N, int ld, float* db) {
   db[n] = s;
 }
 
+// The backward pass of one layer up to its products, in one pass over dL/da: dz = dA gelu'(pre)
+// (dA itself without pre), its BF16 copy, the BF16 transpose the weight gradient's product takes
+// (rows M .. rows_pad zero) and the bias gradient db[n] = sum_m dz[m, n].  A block walks the
+// rows of 32 columns in 32 x 32 tiles; thread (c, q) sums its column's rows q, q + 8, ... in
+// order and the eight sums are added in order.
+// What bounds it: launches and latency (a 256 x 512 layer is 1 MB).  In its place ran GELU
+// backward, the bias gradient (one thread per column, rows in a chain: 17 us), a BF16 copy and a
+// transpose.
+__global__ void __launch_bounds__(256) k_layer_backward(const float* __restrict__ dA, const float* __restrict__ pre,
+                                                        int M, int N, __nv_bfloat16* __restrict__ dz16,
+                                                        __nv_bfloat16* __restrict__ dz16t, int rows_pad,
+                                                        float* __restrict__ db) {
+  __shared__ float tile[2][32][33];
+  __shared__ float sums[8][32];
+  const int c = threadIdx.x % 32, q = threadIdx.x / 32, n0 = blockIdx.x * 32, n = n0 + c;
+  float s = 0.0f;
+  int buffer = 0;
+  for (int m0 = 0; m0 < rows_pad; m0 += 32, buffer ^= 1) {
+    float v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int m = m0 + q + 8 * i;
+      const bool in = m < M && n < N;
+      const size_t at = (size_t)m * N + n;
+      v[i] = in ? dA[at] * (pre ? gelu_grad(pre[at]) : 1.0f) : 0.0f;
+      if (in && dz16) dz16[at] = __float2bfloat16_rn(v[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      s += v[i];
+      tile[buffer][q + 8 * i][c] = v[i];
+    }
+    if (!dz16t) continue;
+    __syncthreads();  // the other buffer is written next: one barrier per tile
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int nn = q + 8 * i;
+      if (n0 + nn < N && m0 + c < rows_pad)
+        dz16t[(size_t)(n0 + nn) * rows_pad + m0 + c] = __float2bfloat16_rn(tile[buffer][c][nn]);
+    }
+  }
+  sums[q][c] = s;
+  __syncthreads();
+  if (q == 0 && n < N) {
+    float total = sums[0][c];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) total += sums[i][c];
+    db[n] = total;
+  }
+}
+
+// The first layer's gradients, K <= 8 inputs: dz = dA gelu'(pre), db[n] = sum_m dz[m, n] and
+// dW[n, k] = sum_m dz[m, n] x[m, k], the factors rounded to BF16 and summed in FP32 as the
+// products are.  32 columns a block, 32 threads a column.
+constexpr int kFirstInputs = 8;
+__global__ void __launch_bounds__(1024) k_first_layer_backward(const float* __restrict__ dA,
+                                                               const float* __restrict__ pre,
+                                                               const float* __restrict__ x, int ldx, int M, int N, int K,
+                                                               float* __restrict__ dW, float* __restrict__ db) {
+  __shared__ float part[32][33];
+  const int c = threadIdx.x % 32, q = threadIdx.x / 32, n = blockIdx.x * 32 + c;
+  float acc[kFirstInputs + 1] = {};
+  if (n < N) {
+    for (int m = q; m < M; m += 32) {
+      const size_t at = (size_t)m * N + n;
+      const float dz = dA[at] * (pre ? gelu_grad(pre[at]) : 1.0f);
+      const float rounded = __bfloat162float(__float2bfloat16_rn(dz));
+      acc[kFirstInputs] += dz;
+#pragma unroll
+      for (int k = 0; k < kFirstInputs; ++k)
+        if (k < K) acc[k] += rounded * __bfloat162float(__float2bfloat16_rn(x[(size_t)m * ldx + k]));
+    }
+  }
+#pragma unroll
+  for (int k = 0; k <= kFirstInputs; ++k) {
+    if (k < kFirstInputs && k >= K) continue;
+    part[q][c] = acc[k];
+    __syncthreads();
+    // thread (q, c) now takes column q's 32 sums
+    float s = part[c][q];
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+    const int nn = blockIdx.x * 32 + q;
+    if (c == 0 && nn < N) {
+      if (k < kFirstInputs) dW[(size_t)nn * K + k] = s;
+      else db[nn] = s;
+    }
+    __syncthreads();
+  }
+}
+
 // dY = 2 (Y - T) / (M N); per-row partial losses, summed by k_loss_total in row order
 __global__ void k_mse(const float* Y, const float* T, int M, int N, float* dY, float* row_loss) {
   const int m = blockIdx.x;
@@ -191,11 +282,12 @@ __global__ void k_mse(const float* Y, const float* T, int M, int N, float* dY, f
   if (threadIdx.x == 0) row_loss[m] = part[0];
 }
 
-__global__ void k_loss_total(const float* row_loss, int M, int N, float* loss) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__global__ void k_loss_total(const float* row_loss, int M, int N, float* loss) {  // one warp
   double s = 0.0;
-  for (int m = 0; m < M; ++m) s += row_loss[m];
-  *loss = (float)(s / ((double)M * (double)N));
+  for (int m = threadIdx.x; m < M; m += 32) s += row_loss[m];
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+  if (threadIdx.x == 0) *loss = (float)(s / ((double)M * (double)N));
 }
 
 // Adam (Kingma & Ba 2015) with bias correction, FP32 master weights
@@ -208,6 +300,36 @@ __global__ void k_adam(float* w, const float* grad, float* m1, float* m2, size_t
     m1[i] = a;
     m2[i] = b;
     w[i] -= lr * (a / c1) / (sqrtf(b / c2) + eps);
+  }
+}
+
+// The same for a list of parameters in one launch: block b works on the tensor q with
+// first[q] <= b < first[q + 1], 1024 elements of it
+constexpr int kMaxParameters = 16;
+struct AdamBatch {
+  float* w[kMaxParameters];
+  const float* grad[kMaxParameters];
+  float* m1[kMaxParameters];
+  float* m2[kMaxParameters];
+  size_t n[kMaxParameters];
+  int first[kMaxParameters + 1];
+  int count;
+};
+__global__ void __launch_bounds__(256) k_adam_batch(const __grid_constant__ AdamBatch p, float lr, float b1, float b2,
+                                                    float eps, float c1, float c2) {
+  int q = 0;
+  while (q + 1 < p.count && (int)blockIdx.x >= p.first[q + 1]) ++q;
+  const size_t from = (size_t)(blockIdx.x - p.first[q]) * 1024 + threadIdx.x;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const size_t at = from + (size_t)i * 256;
+    if (at >= p.n[q]) break;
+    const float gi = p.grad[q][at];
+    const float a = b1 * p.m1[q][at] + (1.0f - b1) * gi;
+    const float b = b2 * p.m2[q][at] + (1.0f - b2) * gi * gi;
+    p.m1[q][at] = a;
+    p.m2[q][at] = b;
+    p.w[q][at] -= lr * (a / c1) / (sqrtf(b / c2) + eps);
   }
 }
 
@@ -312,6 +434,43 @@ sp_status sp_mlp_adam(float* w, const float* grad, float* m1, float* m2, size_t 
   const float c1 = 1.0f - powf(beta1, (float)step), c2 = 1.0f - powf(beta2, (float)step);
   sp::k_adam<<<sp::grid_for(n), 256, 0, (cudaStream_t)stream>>>(w, grad, m1, m2, n, lr, beta1, beta2, eps,
                                                                c1, c2);
+  return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ERR_CUDA;
+}
+
+sp_status sp_mlp_layer_backward(const float* dA, const float* pre, int M, int N, void* dz16, void* dz16t,
+                                int rows_pad, float* db, void* stream) {
+  if (!dA || !db || M < 0 || N < 0 || rows_pad < M) return SP_ERR_ARGUMENT;
+  if (!N) return SP_OK;
+  sp::k_layer_backward<<<(N + 31) / 32, 256, 0, (cudaStream_t)stream>>>(
+      dA, pre, M, N, static_cast<__nv_bfloat16*>(dz16), static_cast<__nv_bfloat16*>(dz16t), rows_pad, db);
+  return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ERR_CUDA;
+}
+
+sp_status sp_mlp_first_layer_backward(const float* dA, const float* pre, const float* x, int ldx, int M, int N, int K,
+                                      float* dW, float* db, void* stream) {
+  if (!dA || !x || !dW || !db || M < 0 || N < 0 || K < 1 || K > sp::kFirstInputs || ldx < K) return SP_ERR_ARGUMENT;
+  if (!N) return SP_OK;
+  sp::k_first_layer_backward<<<(N + 31) / 32, 1024, 0, (cudaStream_t)stream>>>(dA, pre, x, ldx, M, N, K, dW, db);
+  return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ERR_CUDA;
+}
+
+sp_status sp_mlp_adam_batch(int count, float* const* w, const float* const* grad, float* const* m1, float* const* m2,
+                            const size_t* n, float lr, float beta1, float beta2, float eps, int step, void* stream) {
+  if (count < 1 || count > sp::kMaxParameters || !w || !grad || !m1 || !m2 || !n || step < 1) return SP_ERR_ARGUMENT;
+  sp::AdamBatch p{};
+  p.count = count;
+  for (int q = 0; q < count; ++q) {
+    if (!w[q] || !grad[q] || !m1[q] || !m2[q] || n[q] > ((size_t)1 << 40)) return SP_ERR_ARGUMENT;
+    p.w[q] = w[q];
+    p.grad[q] = grad[q];
+    p.m1[q] = m1[q];
+    p.m2[q] = m2[q];
+    p.n[q] = n[q];
+    p.first[q + 1] = p.first[q] + (int)((n[q] + 1023) / 1024);
+  }
+  if (!p.first[count]) return SP_OK;
+  const float c1 = 1.0f - powf(beta1, (float)step), c2 = 1.0f - powf(beta2, (float)step);
+  sp::k_adam_batch<<<p.first[count], 256, 0, (cudaStream_t)stream>>>(p, lr, beta1, beta2, eps, c1, c2);
   return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ERR_CUDA;
 }
 

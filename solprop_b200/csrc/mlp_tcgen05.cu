@@ -319,6 +319,49 @@ __global__ void k_transpose_bf16(const T* src, int ld_src, int rows, int cols, _
   }
 }
 
+// Several matrices in one launch: of each FP32 (or BF16) rows x cols matrix a BF16 copy with rows
+// of cols_out (zero-padded) and / or a BF16 transpose with rows of rows_pad (zero-padded).  Block
+// b takes the 32 x 32 tile b - first[q] of matrix q; the source is read once.
+constexpr int kMaxConversions = 8;
+struct ConvertBatch {
+  const void* src[kMaxConversions];
+  __nv_bfloat16* copy[kMaxConversions];
+  __nv_bfloat16* transpose[kMaxConversions];
+  int rows[kMaxConversions], cols[kMaxConversions], ld[kMaxConversions];
+  int cols_out[kMaxConversions], rows_pad[kMaxConversions], tiles_c[kMaxConversions];
+  int first[kMaxConversions + 1];
+  int count;
+};
+template <class T>
+__global__ void __launch_bounds__(256) k_convert_bf16(const __grid_constant__ ConvertBatch p) {
+  __shared__ __nv_bfloat16 tile[32][34];
+  int q = 0;
+  while (q + 1 < p.count && (int)blockIdx.x >= p.first[q + 1]) ++q;
+  const int b = blockIdx.x - p.first[q], r0 = b / p.tiles_c[q] * 32, c0 = b % p.tiles_c[q] * 32;
+  const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
+  const T* src = static_cast<const T*>(p.src[q]);
+  __nv_bfloat16* copy = p.copy[q];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = r0 + ty + 8 * i, c = c0 + tx;
+    __nv_bfloat16 v = __float2bfloat16_rn(0.0f);
+    if (r < p.rows[q] && c < p.cols[q]) {
+      if constexpr (sizeof(T) == 4) v = __float2bfloat16_rn(src[(size_t)r * p.ld[q] + c]);
+      else v = src[(size_t)r * p.ld[q] + c];
+    }
+    if (copy && r < p.rows[q] && c < p.cols_out[q]) copy[(size_t)r * p.cols_out[q] + c] = v;
+    tile[ty + 8 * i][tx] = v;
+  }
+  __nv_bfloat16* transpose = p.transpose[q];
+  if (!transpose) return;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int c = c0 + ty + 8 * i, r = r0 + tx;
+    if (c < p.cols[q] && r < p.rows_pad[q]) transpose[(size_t)c * p.rows_pad[q] + r] = tile[tx][ty + 8 * i];
+  }
+}
+
 // a rows x cols BF16 matrix (row pitch ld elements) as 2-D tiles of box_rows x 64
 bool make_map(CUtensorMap* map, const void* base, int rows, int cols, int ld, int box_rows) {
   return tc::make_bf16_map(map, base, rows, cols, ld, box_rows, kTK);
@@ -392,6 +435,36 @@ sp_status sp_mlp_transpose_bf16(const void* src, int src_bf16, int ld_src, int r
   else
     sp::k_transpose_bf16<float><<<grid, block, 0, (cudaStream_t)stream>>>(
         static_cast<const float*>(src), ld_src, rows, cols, static_cast<__nv_bfloat16*>(dst), ld_dst, rows_pad);
+  return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ERR_CUDA;
+}
+
+sp_status sp_mlp_convert_batch(int count, int src_bf16, const void* const* src, const int* rows, const int* cols,
+                               const int* ld, void* const* copy, const int* cols_out, void* const* transpose,
+                               const int* rows_pad, void* stream) {
+  using namespace sp;
+  if (count < 1 || count > kMaxConversions || !src || !rows || !cols || !ld || !copy || !cols_out || !transpose ||
+      !rows_pad)
+    return SP_ERR_ARGUMENT;
+  ConvertBatch p{};
+  p.count = count;
+  for (int q = 0; q < count; ++q) {
+    if (!src[q] || rows[q] < 0 || cols[q] < 0 || ld[q] < cols[q]) return SP_ERR_ARGUMENT;
+    if ((copy[q] && cols_out[q] < cols[q]) || (transpose[q] && rows_pad[q] < rows[q])) return SP_ERR_ARGUMENT;
+    p.src[q] = src[q];
+    p.copy[q] = static_cast<__nv_bfloat16*>(copy[q]);
+    p.transpose[q] = static_cast<__nv_bfloat16*>(transpose[q]);
+    p.rows[q] = rows[q];
+    p.cols[q] = cols[q];
+    p.ld[q] = ld[q];
+    p.cols_out[q] = cols_out[q];
+    p.rows_pad[q] = rows_pad[q];
+    const int r = transpose[q] ? rows_pad[q] : rows[q], c = copy[q] ? cols_out[q] : cols[q];
+    p.tiles_c[q] = (c + 31) / 32;
+    p.first[q + 1] = p.first[q] + p.tiles_c[q] * ((r + 31) / 32);
+  }
+  if (!p.first[count]) return SP_OK;
+  if (src_bf16) k_convert_bf16<__nv_bfloat16><<<p.first[count], 256, 0, (cudaStream_t)stream>>>(p);
+  else k_convert_bf16<float><<<p.first[count], 256, 0, (cudaStream_t)stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ERR_CUDA;
 }
 

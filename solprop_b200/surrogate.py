@@ -132,6 +132,29 @@ def transpose_bf16(x, rows_pad: int):
     return out
 
 
+def convert_batch(xs, copies=None, transposes=None):
+    """BF16 copies (rows zero-padded to ``copies[q]`` columns) and transposes (zero-padded to
+    ``transposes[q]`` source rows) of up to eight FP32 or BF16 matrices in one launch, either
+    list None; returns the two lists."""
+    import torch
+
+    n = len(xs)
+    new = lambda rows, cols, x: torch.empty((rows, cols), dtype=torch.bfloat16, device=x.device)  # noqa: E731
+    out = [new(x.shape[0], c, x) for x, c in zip(xs, copies)] if copies else None
+    out_t = [new(x.shape[1], r, x) for x, r in zip(xs, transposes)] if transposes else None
+    ints = lambda v: (C.c_int * n)(*v)  # noqa: E731
+    none = [None] * n
+    _check(_bind().sp_mlp_convert_batch(
+        n, int(xs[0].dtype == torch.bfloat16), _pointers(xs), ints(x.shape[0] for x in xs),
+        ints(x.shape[1] for x in xs), ints(x.stride(0) for x in xs), _pointers(out or none), ints(copies or [0] * n),
+        _pointers(out_t or none), ints(transposes or [0] * n), None))
+    return out, out_t
+
+
+def _pointers(tensors):
+    return (C.c_void_p * len(tensors))(*[None if t is None else t.data_ptr() for t in tensors])
+
+
 def _pad64(n: int) -> int:
     return -(-n // 64) * 64
 
@@ -245,11 +268,14 @@ class Perceptron:
         activations in BF16 (epilogue 3).  Returns the output, the cache and the status."""
         import torch
 
-        a = to_bf16(x, _pad64(x.shape[1]))
+        inputs = [x, *self.weights]
+        if x.dtype == torch.float32 and len(inputs) <= 8:
+            (a, *w16s), _ = convert_batch(inputs, [_pad64(t.shape[1]) for t in inputs])
+        else:
+            a, *w16s = [to_bf16(t, _pad64(t.shape[1])) for t in inputs]
         cache = []
         last = len(self.weights) - 1
-        for i, (w, b) in enumerate(zip(self.weights, self.biases)):
-            w16 = to_bf16(w, _pad64(w.shape[1]))
+        for i, (w, w16, b) in enumerate(zip(self.weights, w16s, self.biases)):
             if i == last:
                 out = torch.empty((a.shape[0], w.shape[0]), dtype=torch.float32, device=self.device)
                 status = gemm_tc(a, w16, out=out, bias=b, epilogue=1, status=status)
@@ -265,32 +291,43 @@ class Perceptron:
         """dW, db of every layer from dL/dy on the tcgen05 products: the weight gradient
         dz^T a and the input gradient dz W as products C = A W^T of BF16 transposes (the
         batch zero-padded to a multiple of 64); the first layer's 6-input weight gradient,
-        below the products' 256-column tiles, on the FP32 path.  Returns (grads, status)."""
+        below the products' 256-column tiles, in a kernel of its own.  Each layer's dz, its
+        copies and its bias gradient come from one pass, the transposes of the weights and of
+        the activations from one launch each, and the weight gradients of one shape share a
+        launch.  Returns (grads, status)."""
         import torch
 
         lib = _bind()
-        grads = [None] * len(self.params)
+        grads = [torch.empty_like(p) for p in self.params]
+        if status is None:
+            status = torch.zeros(1, dtype=torch.int32, device=dy.device)
+        last = len(self.weights) - 1
+        m, rows = dy.shape[0], _pad64(dy.shape[0])
+        upper = range(1, last + 1)
+        w16t = convert_batch([self.weights[i] for i in upper], None, [self.weights[i].shape[0] for i in upper])[1]
+        a16t = convert_batch([cache[i][0] for i in upper], None, [rows] * last)[1]
         g = dy
-        rows = _pad64(dy.shape[0])
-        for i in range(len(self.weights) - 1, -1, -1):
-            a, pre = cache[i]
-            w = self.weights[i]
-            if pre is not None:
-                dz = torch.empty_like(g)
-                _check(lib.sp_mlp_gelu_backward(_ptr(g), _ptr(pre), _ptr(dz), g.numel(), None))
-                g = dz
-            dw = torch.empty_like(w)
-            if w.shape[1] % 256 == 0:
-                status = gemm_tc(transpose_bf16(g, rows), transpose_bf16(a, rows), out=dw, status=status)
-            else:
-                gemm(g, a, dw, trans_a=True)
-            db = torch.empty_like(self.biases[i])
-            _check(lib.sp_mlp_bias_grad(_ptr(g), g.shape[0], g.shape[1], _ptr(db), None))
-            grads[2 * i], grads[2 * i + 1] = dw, db
-            if i:
-                da = torch.empty((g.shape[0], w.shape[1]), dtype=torch.float32, device=self.device)
-                status = gemm_tc(to_bf16(g, g.shape[1]), transpose_bf16(w, w.shape[0]), out=da, status=status)
-                g = da
+        dz16t = [None] * (last + 1)
+        for i in range(last, 0, -1):
+            pre = cache[i][1]
+            n, k = self.weights[i].shape
+            dz16 = torch.empty((m, n), dtype=torch.bfloat16, device=self.device)
+            dz16t[i] = torch.empty((n, rows), dtype=torch.bfloat16, device=self.device)
+            _check(lib.sp_mlp_layer_backward(_ptr(g), None if pre is None else _ptr(pre), m, n, _ptr(dz16),
+                                             _ptr(dz16t[i]), rows, _ptr(grads[2 * i + 1]), None))
+            g = torch.empty((m, k), dtype=torch.float32, device=self.device)
+            status = gemm_tc(dz16, w16t[i - 1], out=g, status=status)
+        # the weight gradients, the layers of one shape together
+        shapes = {}
+        for i in upper:
+            shapes.setdefault(self.weights[i].shape, []).append(i)
+        for layers in shapes.values():
+            status = gemm_tc_batch([dz16t[i] for i in layers], [a16t[i - 1] for i in layers],
+                                   outs=[grads[2 * i] for i in layers], status=status)
+        x, pre = cache[0]
+        n, k = self.weights[0].shape
+        _check(lib.sp_mlp_first_layer_backward(_ptr(g), None if pre is None else _ptr(pre), _ptr(x), x.stride(0), m, n,
+                                               k, _ptr(grads[0]), _ptr(grads[1]), None))
         return grads, status
 
     def gradients(self, cache, dy):
@@ -321,9 +358,9 @@ class Perceptron:
     def adam(self, grads, lr: float, betas=(0.9, 0.999), eps: float = 1e-8):
         lib = _bind()
         self.step += 1
-        for p, g, m1, m2 in zip(self.params, grads, self.m1, self.m2):
-            _check(lib.sp_mlp_adam(_ptr(p), _ptr(g), _ptr(m1), _ptr(m2), p.numel(), lr, betas[0],
-                                   betas[1], eps, self.step, None))
+        sizes = (C.c_size_t * len(grads))(*[p.numel() for p in self.params])
+        _check(lib.sp_mlp_adam_batch(len(grads), _pointers(self.params), _pointers(grads), _pointers(self.m1),
+                                     _pointers(self.m2), sizes, lr, betas[0], betas[1], eps, self.step, None))
 
 
 def mse(y, t):
