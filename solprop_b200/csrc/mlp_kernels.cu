@@ -172,53 +172,51 @@ __global__ void k_bias_grad(const float* dZ, int M, int N, int ld, float* db) {
 
 // The backward pass of one layer up to its products, in one pass over dL/da: dz = dA gelu'(pre)
 // (dA itself without pre), its BF16 copy, the BF16 transpose the weight gradient's product takes
-// (rows M .. rows_pad zero) and the bias gradient db[n] = sum_m dz[m, n].  A block walks the
-// rows of 32 columns in 32 x 32 tiles; thread (c, q) sums its column's rows q, q + 8, ... in
-// order and the eight sums are added in order.
-// What bounds it: launches and latency (a 256 x 512 layer is 1 MB).  In its place ran GELU
-// backward, the bias gradient (one thread per column, rows in a chain: 17 us), a BF16 copy and a
-// transpose.
-__global__ void __launch_bounds__(256) k_layer_backward(const float* __restrict__ dA, const float* __restrict__ pre,
-                                                        int M, int N, __nv_bfloat16* __restrict__ dz16,
-                                                        __nv_bfloat16* __restrict__ dz16t, int rows_pad,
-                                                        float* __restrict__ db) {
+// (rows M .. rows_pad zero) and the bias gradient db[n] = sum_m dz[m, n].  A block of 32 x 32
+// threads takes 32 columns, eight 32-row tiles at a time, all their loads issued first; thread
+// (c, q) sums its column's rows q, q + 32, ... in order and the 32 sums are added as a tree.
+// What bounds it: latency (a 256 x 512 layer is 1 MB).  ncu, 256 rows: 8 us; in its place ran
+// GELU backward, the bias gradient (one thread per column, rows in a chain: 17 us), a BF16 copy
+// and a transpose, 28 us and four launches.
+constexpr int kBackTiles = 8;
+__global__ void __launch_bounds__(1024) k_layer_backward(const float* __restrict__ dA, const float* __restrict__ pre,
+                                                         int M, int N, __nv_bfloat16* __restrict__ dz16,
+                                                         __nv_bfloat16* __restrict__ dz16t, int rows_pad,
+                                                         float* __restrict__ db) {
   __shared__ float tile[2][32][33];
-  __shared__ float sums[8][32];
   const int c = threadIdx.x % 32, q = threadIdx.x / 32, n0 = blockIdx.x * 32, n = n0 + c;
   float s = 0.0f;
-  int buffer = 0;
-  for (int m0 = 0; m0 < rows_pad; m0 += 32, buffer ^= 1) {
-    float v[4];
+  for (int base = 0; base < rows_pad; base += 32 * kBackTiles) {
+    float v[kBackTiles], z[kBackTiles];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int m = m0 + q + 8 * i;
+    for (int i = 0; i < kBackTiles; ++i) {
+      const int m = base + 32 * i + q;
       const bool in = m < M && n < N;
-      const size_t at = (size_t)m * N + n;
-      v[i] = in ? dA[at] * (pre ? gelu_grad(pre[at]) : 1.0f) : 0.0f;
-      if (in && dz16) dz16[at] = __float2bfloat16_rn(v[i]);
+      v[i] = in ? dA[(size_t)m * N + n] : 0.0f;
+      z[i] = in && pre ? pre[(size_t)m * N + n] : 0.0f;
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      s += v[i];
-      tile[buffer][q + 8 * i][c] = v[i];
-    }
-    if (!dz16t) continue;
-    __syncthreads();  // the other buffer is written next: one barrier per tile
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int nn = q + 8 * i;
-      if (n0 + nn < N && m0 + c < rows_pad)
-        dz16t[(size_t)(n0 + nn) * rows_pad + m0 + c] = __float2bfloat16_rn(tile[buffer][c][nn]);
+    for (int i = 0; i < kBackTiles; ++i) {
+      const int m0 = base + 32 * i, m = m0 + q;
+      if (m0 >= rows_pad) break;  // uniform
+      const float dz = pre ? v[i] * gelu_grad(z[i]) : v[i];
+      s += dz;
+      if (dz16 && m < M && n < N) dz16[(size_t)m * N + n] = __float2bfloat16_rn(dz);
+      if (!dz16t) continue;
+      tile[i & 1][q][c] = dz;
+      __syncthreads();  // the other buffer is written next: one barrier per tile
+      if (n0 + q < N && m0 + c < rows_pad)
+        dz16t[(size_t)(n0 + q) * rows_pad + m0 + c] = __float2bfloat16_rn(tile[i & 1][c][q]);
     }
   }
-  sums[q][c] = s;
   __syncthreads();
-  if (q == 0 && n < N) {
-    float total = sums[0][c];
+  tile[0][q][c] = s;
+  __syncthreads();
+  // thread (q, c) now takes column q's 32 sums
+  float total = tile[0][c][q];
 #pragma unroll
-    for (int i = 1; i < 8; ++i) total += sums[i][c];
-    db[n] = total;
-  }
+  for (int d = 16; d > 0; d >>= 1) total += __shfl_xor_sync(0xffffffffu, total, d);
+  if (c == 0 && n0 + q < N) db[n0 + q] = total;
 }
 
 // The first layer's gradients, K <= 8 inputs: dz = dA gelu'(pre), db[n] = sum_m dz[m, n] and
@@ -441,7 +439,7 @@ sp_status sp_mlp_layer_backward(const float* dA, const float* pre, int M, int N,
                                 int rows_pad, float* db, void* stream) {
   if (!dA || !db || M < 0 || N < 0 || rows_pad < M) return SP_ERR_ARGUMENT;
   if (!N) return SP_OK;
-  sp::k_layer_backward<<<(N + 31) / 32, 256, 0, (cudaStream_t)stream>>>(
+  sp::k_layer_backward<<<(N + 31) / 32, 1024, 0, (cudaStream_t)stream>>>(
       dA, pre, M, N, static_cast<__nv_bfloat16*>(dz16), static_cast<__nv_bfloat16*>(dz16t), rows_pad, db);
   return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ERR_CUDA;
 }

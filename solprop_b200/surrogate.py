@@ -134,11 +134,15 @@ def transpose_bf16(x, rows_pad: int):
 
 def convert_batch(xs, copies=None, transposes=None):
     """BF16 copies (rows zero-padded to ``copies[q]`` columns) and transposes (zero-padded to
-    ``transposes[q]`` source rows) of up to eight FP32 or BF16 matrices in one launch, either
-    list None; returns the two lists."""
+    ``transposes[q]`` source rows) of FP32 or BF16 matrices, eight to a launch, either list
+    None; returns the two lists."""
     import torch
 
     n = len(xs)
+    if n > 8:
+        head = convert_batch(xs[:8], copies and copies[:8], transposes and transposes[:8])
+        tail = convert_batch(xs[8:], copies and copies[8:], transposes and transposes[8:])
+        return tuple(None if a is None else a + b for a, b in zip(head, tail))
     new = lambda rows, cols, x: torch.empty((rows, cols), dtype=torch.bfloat16, device=x.device)  # noqa: E731
     out = [new(x.shape[0], c, x) for x, c in zip(xs, copies)] if copies else None
     out_t = [new(x.shape[1], r, x) for x, r in zip(xs, transposes)] if transposes else None
@@ -269,10 +273,7 @@ class Perceptron:
         import torch
 
         inputs = [x, *self.weights]
-        if x.dtype == torch.float32 and len(inputs) <= 8:
-            (a, *w16s), _ = convert_batch(inputs, [_pad64(t.shape[1]) for t in inputs])
-        else:
-            a, *w16s = [to_bf16(t, _pad64(t.shape[1])) for t in inputs]
+        (a, *w16s), _ = convert_batch(inputs, [_pad64(t.shape[1]) for t in inputs])
         cache = []
         last = len(self.weights) - 1
         for i, (w, w16, b) in enumerate(zip(self.weights, w16s, self.biases)):
@@ -321,13 +322,20 @@ class Perceptron:
         shapes = {}
         for i in upper:
             shapes.setdefault(self.weights[i].shape, []).append(i)
-        for layers in shapes.values():
-            status = gemm_tc_batch([dz16t[i] for i in layers], [a16t[i - 1] for i in layers],
-                                   outs=[grads[2 * i] for i in layers], status=status)
+        for alike in shapes.values():
+            for layers in (alike[s:s + 8] for s in range(0, len(alike), 8)):
+                status = gemm_tc_batch([dz16t[i] for i in layers], [a16t[i - 1] for i in layers],
+                                       outs=[grads[2 * i] for i in layers], status=status)
         x, pre = cache[0]
         n, k = self.weights[0].shape
-        _check(lib.sp_mlp_first_layer_backward(_ptr(g), None if pre is None else _ptr(pre), _ptr(x), x.stride(0), m, n,
-                                               k, _ptr(grads[0]), _ptr(grads[1]), None))
+        if k <= 8:
+            _check(lib.sp_mlp_first_layer_backward(_ptr(g), None if pre is None else _ptr(pre), _ptr(x), x.stride(0),
+                                                   m, n, k, _ptr(grads[0]), _ptr(grads[1]), None))
+        else:
+            if pre is not None:
+                _check(lib.sp_mlp_gelu_backward(_ptr(g), _ptr(pre), _ptr(g), g.numel(), None))
+            gemm(g, x, grads[0], trans_a=True)
+            _check(lib.sp_mlp_bias_grad(_ptr(g), m, n, _ptr(grads[1]), None))
         return grads, status
 
     def gradients(self, cache, dy):
@@ -358,9 +366,12 @@ class Perceptron:
     def adam(self, grads, lr: float, betas=(0.9, 0.999), eps: float = 1e-8):
         lib = _bind()
         self.step += 1
-        sizes = (C.c_size_t * len(grads))(*[p.numel() for p in self.params])
-        _check(lib.sp_mlp_adam_batch(len(grads), _pointers(self.params), _pointers(grads), _pointers(self.m1),
-                                     _pointers(self.m2), sizes, lr, betas[0], betas[1], eps, self.step, None))
+        for s in range(0, len(grads), 16):
+            part = slice(s, s + 16)
+            sizes = (C.c_size_t * len(grads[part]))(*[p.numel() for p in self.params[part]])
+            _check(lib.sp_mlp_adam_batch(len(sizes), _pointers(self.params[part]), _pointers(grads[part]),
+                                         _pointers(self.m1[part]), _pointers(self.m2[part]), sizes, lr, betas[0],
+                                         betas[1], eps, self.step, None))
 
 
 def mse(y, t):
