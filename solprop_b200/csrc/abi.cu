@@ -298,7 +298,7 @@ struct sp_workspace {
   DevBuf<double2> raman_spectrum;  // field-grid Raman: the damped kernel's spectrum (n_to + 1)
   DevBuf<int> raman_scale;         // the envelope products' mixed form: the spectra's powers of two
   // the envelope products' nodes: the spectra and twiddles in the register transform's order
-  DevBuf<double2> raman_table, outer_twiddles, inner_twiddles, row_outer, row_inner;
+  DevBuf<double2> raman_table, row_outer, row_inner;
   DevBuf<double2> env_scratch;      // the envelope products' FP64 rows above 8192 samples: 1.5 n_to per row
   DevBuf<double2> raman_scratch;    // ... and the Raman kernel's spectra
   DevBuf<ChannelTableT<double>> channels;  // a mixture's plasma channels (rate_coeff holds their tables)
@@ -316,7 +316,7 @@ struct sp_workspace {
     DevBuf<float> t_window, t_window_d, synthesis, projection, rate_coeff, taps, proj;
     DevBuf<float> node_field, node_streams;
     DevBuf<ChannelTableT<float>> channels;
-    DevBuf<float2> env_twiddles, raman_table, outer_twiddles, inner_twiddles, row_outer, row_inner;
+    DevBuf<float2> env_twiddles, raman_table, row_outer, row_inner;
   } f32;
   DevBuf<unsigned char> active, norm;
   DevBuf<StageScalarsDev> stage;   // kStageSlots slots
@@ -714,10 +714,8 @@ static EnvModalArgsT<R> env_modal_args(const sp_workspace* ws, const double2* la
   if constexpr (sizeof(R) == 8) {
     ea.twiddles_r = ws->env_twiddles.p;
     ea.raman_table = ws->raman_table.p;
-    ea.row_outer_r = ws->row_outer.p;
-    ea.row_inner_r = ws->row_inner.p;
-    ea.outer_twiddles = ws->outer_twiddles.p;
-    ea.inner_twiddles = ws->inner_twiddles.p;
+    ea.outer_twiddles = ws->row_outer.p;
+    ea.inner_twiddles = ws->row_inner.p;
     ea.node_field = ws->node_field.p;
     ea.node_streams = ws->node_streams.p;
     ea.projected = ws->proj.p;
@@ -725,10 +723,8 @@ static EnvModalArgsT<R> env_modal_args(const sp_workspace* ws, const double2* la
   } else {
     ea.twiddles_r = ws->f32.env_twiddles.p;
     ea.raman_table = ws->f32.raman_table.p;
-    ea.row_outer_r = ws->f32.row_outer.p;
-    ea.row_inner_r = ws->f32.row_inner.p;
-    ea.outer_twiddles = ws->f32.outer_twiddles.p;
-    ea.inner_twiddles = ws->f32.inner_twiddles.p;
+    ea.outer_twiddles = ws->f32.row_outer.p;
+    ea.inner_twiddles = ws->f32.row_inner.p;
     ea.raman_scale = ws->raman_scale.p;
     ea.node_field = ws->f32.node_field.p;
     ea.node_streams = ws->f32.node_streams.p;
@@ -1087,43 +1083,28 @@ static void build_workspace(sp_workspace* ws) {
     if (d.raman_enabled && (d.grid_kind == 0 || ws->gemm))
       ws->raman_spectrum.alloc((size_t)P.raman_kernels * (d.n_to + 1));
     if (d.grid_kind == 1) {
-      // the register transform's tables, for the nodes' rows and the columns' (FP64 rows above
-      // kMaxEnvelopeRowF64 take the long form)
+      // the register transform's tables (FP64 rows above kMaxEnvelopeRowF64 take the long form)
       const bool mixed = ws->precision == SP_PRECISION_MIXED, rows64 = d.n_to <= kMaxEnvelopeRowF64;
       const size_t table = d.raman_enabled && ws->gemm ? (size_t)2 * P.raman_kernels * d.n_to : 0;
       std::vector<double2> outer, inner;
-      auto wide = [&](const std::vector<double2>& v, DevBuf<double2>& dst) {
-        dst.upload(v.data(), v.size(), s);
-        CUDA_CHECK(cudaStreamSynchronize(s));  // the host copy is overwritten or goes with its scope
-      };
-      auto narrow = [&](const std::vector<double2>& v, DevBuf<float2>& dst) {
-        std::vector<float2> f(v.size());
-        for (size_t m = 0; m < v.size(); ++m) f[m] = make_float2((float)v[m].x, (float)v[m].y);
-        dst.upload(f.data(), f.size(), s);
-        CUDA_CHECK(cudaStreamSynchronize(s));
-      };
-      row_twiddles(d.n_to, env_column_log_v(d.n_to), tw2, outer, inner);
+      row_twiddles(d.n_to, tw2, outer, inner);
       if (rows64) {
-        wide(outer, ws->row_outer);
-        wide(inner, ws->row_inner);
+        ws->row_outer.upload(outer.data(), outer.size(), s);
+        ws->row_inner.upload(inner.data(), inner.size(), s);
+        if (!mixed && table) ws->raman_table.alloc(table);
+        CUDA_CHECK(cudaStreamSynchronize(s));  // the host copies go with this scope
       }
       if (mixed) {
+        auto narrow = [&](const std::vector<double2>& v, DevBuf<float2>& dst) {
+          std::vector<float2> f(v.size());
+          for (size_t m = 0; m < v.size(); ++m) f[m] = make_float2((float)v[m].x, (float)v[m].y);
+          dst.upload(f.data(), f.size(), s);
+          CUDA_CHECK(cudaStreamSynchronize(s));  // the host copy goes with this scope
+        };
         narrow(outer, ws->f32.row_outer);
         narrow(inner, ws->f32.row_inner);
+        if (table) ws->f32.raman_table.alloc(table);
         ws->raman_scale.alloc(2);
-      }
-      if (table) {
-        if (env_node_log_v(d.n_to) != env_column_log_v(d.n_to))
-          row_twiddles(d.n_to, env_node_log_v(d.n_to), tw2, outer, inner);
-        if (mixed) {
-          narrow(outer, ws->f32.outer_twiddles);
-          narrow(inner, ws->f32.inner_twiddles);
-          ws->f32.raman_table.alloc(table);
-        } else if (rows64) {
-          wide(outer, ws->outer_twiddles);
-          wide(inner, ws->inner_twiddles);
-          ws->raman_table.alloc(table);
-        }
       }
     }
     if (d.grid_kind == 1 && ws->gemm && d.n_to > kMaxEnvelopeRowF64) {

@@ -36,13 +36,10 @@ constexpr int kEnvThreads = 1024;
 
 // A column's (or kernel's) transform is one CTA's chain of passes, run once: what bounds it is
 // latency, the instructions' own fetch included, so its threads hold 16 points where the three
-// passes allow it (half the unrolled code of 32, twice the warps).  30 columns of 4 096 and two
+// passes allow it (fft_regs.cuh).  30 columns of 4 096 and two
 // Raman kernels, ncu: the inverse and the kernels' spectra 32.6 + 28.6 us with shared-memory
 // radix-4 transforms in launches of their own -> 32.4 us, the FP32 forward 14.7 -> 13.4 (with
 // 32 points per thread 28.6); FP64 columns of 8 192: 66 + 46 -> 57 us, the forward 34 us.
-constexpr int column_log_v(int log_n) { return log_n <= 12 ? 4 : 5; }
-template <class C, int LOGN>
-using ColumnRow = regs::Row<C, LOGN, column_log_v(LOGN)>;
 
 // The Raman kernels' spectra in k_env_pairs' order (rows of up to 8 192; longer ones take
 // k_raman_kernel and k_raman_table): one CTA per kernel and half p transforms the damped
@@ -52,7 +49,7 @@ using ColumnRow = regs::Row<C, LOGN, column_log_v(LOGN)>;
 template <class R, int LOGN>
 __device__ __forceinline__ void raman_row(const EnvModalArgsT<R>& a, const RamanArgs& ra, cplx<R>* table, int kernel,
                                           int half, double* plane) {
-  using Row = ColumnRow<double2, LOGN>;
+  using Row = regs::Row<double2, LOGN>;
   constexpr int n = Row::N, T = Row::T, V = Row::V;
   const int t0 = threadIdx.x;
   double2 x[V];
@@ -85,7 +82,7 @@ __device__ __forceinline__ void raman_row(const EnvModalArgsT<R>& a, const Raman
   cplx<R>* out = table + ((size_t)kernel * 2 + half) * n;
 #pragma unroll
   for (int e = 0; e < V; ++e)
-    out[regs::Row<cplx<R>, LOGN>::place(Row::bin(t0, e))] = to_c<cplx<R>>(cscale(f, x[e]));
+    out[e * T + t0] = to_c<cplx<R>>(cscale(f, x[e]));
 }
 
 // The inverse transform of a column: the padded spectrum is gathered in the register
@@ -95,9 +92,9 @@ __device__ __forceinline__ void raman_row(const EnvModalArgsT<R>& a, const Raman
 // The Raman kernels' spectra take their CTAs of the same launch, ahead of the columns': they
 // are as long a chain, and nothing of them depends on the field.
 template <class R, int LOGN>
-__global__ void __launch_bounds__(ColumnRow<double2, LOGN>::T)
+__global__ void __launch_bounds__(regs::Row<double2, LOGN>::T)
     k_env_inverse(EnvModalArgsT<R> a, RamanArgs ra, cplx<R>* table, int raman_rows) {
-  using Row = ColumnRow<double2, LOGN>;
+  using Row = regs::Row<double2, LOGN>;
   constexpr int n = Row::N, T = Row::T, V = Row::V;
   extern __shared__ __align__(16) double ei_plane[];
   if ((int)blockIdx.x < raman_rows) {
@@ -221,6 +218,13 @@ __device__ __forceinline__ void node_output(const EnvModalArgsT<R>& a, int nc, d
   }
 }
 
+// resident CTAs: the rows fill the registers of an SM (V points of 8 or 16 bytes and as much again)
+template <class R, int LOGN>
+constexpr int pairs_resident() {
+  using Row = regs::Row<cplx<R>, LOGN>;
+  return (sizeof(R) == 4 ? 16384 : 8192) / Row::V / Row::T;
+}
+
 // The nodes' responses with Raman, one CTA per two nodes A and B.  A convolution with a real
 // kernel takes two real drives as one complex row: the trace drives of A and B together
 // (drive |a|^2 / 2, or |a_x|^2 / 2 + |a_y|^2 / 2 of two field components), then, where the
@@ -238,7 +242,7 @@ __device__ __forceinline__ void node_output(const EnvModalArgsT<R>& a, int nc, d
 // 16 384 nodes of two components, rows of 16 384, FP32: 33.0 -> 7 ms; 2 025 nodes, rows of
 // 8 192, FP64: 2.78 -> 1.0 ms.
 template <class R, int LOGN>
-__global__ void __launch_bounds__(regs::Row<cplx<R>, LOGN>::T, (sizeof(R) == 4 ? 512 : 256) / regs::Row<cplx<R>, LOGN>::T)
+__global__ void __launch_bounds__(regs::Row<cplx<R>, LOGN>::T, pairs_resident<R, LOGN>())
     k_env_pairs(EnvModalArgsT<R> a, int n_nodes) {
   using C = cplx<R>;
   using Row = regs::Row<C, LOGN>;
@@ -349,16 +353,16 @@ __global__ void __launch_bounds__(256) k_raman_table(const double2* __restrict__
 
 // The forward transform of a projected column, its bins scattered to the cropped spectrum
 template <class R, int LOGN>
-__global__ void __launch_bounds__(ColumnRow<cplx<R>, LOGN>::T) k_env_forward(EnvModalArgsT<R> a) {
+__global__ void __launch_bounds__(regs::Row<cplx<R>, LOGN>::T) k_env_forward(EnvModalArgsT<R> a) {
   using C = cplx<R>;
-  using Row = ColumnRow<C, LOGN>;
+  using Row = regs::Row<C, LOGN>;
   extern __shared__ __align__(16) unsigned char ef_raw[];
   const int col = blockIdx.x, t0 = threadIdx.x;
   const C* row = reinterpret_cast<const C*>(a.projected) + (size_t)col * Row::N + t0;
   C x[Row::V];
 #pragma unroll
   for (int r = 0; r < Row::V; ++r) x[r] = row[r * Row::T];
-  Row::forward(x, reinterpret_cast<R*>(ef_raw), a.row_outer_r, a.row_inner_r, 0);
+  Row::forward(x, reinterpret_cast<R*>(ef_raw), a.outer_twiddles, a.inner_twiddles, 0);
   C* spectra = a.spectra + (size_t)col * a.n_omega;
 #pragma unroll
   for (int e = 0; e < Row::V; ++e) {
@@ -542,7 +546,7 @@ static cudaError_t with_row(int log_n, F&& f) {
 }
 
 template <class C, int LOGN>
-constexpr size_t plane_smem() { return ColumnRow<C, LOGN>::kPlane * sizeof(typename ColumnRow<C, LOGN>::R); }
+constexpr size_t plane_smem() { return regs::Row<C, LOGN>::kPlane * sizeof(typename regs::Row<C, LOGN>::R); }
 
 cudaError_t configure_env_modal_kernels() {
   const int row = (int)(kMaxEnvelopeRowF64 * sizeof(double2));  // half a long FP64 row
@@ -574,13 +578,10 @@ cudaError_t configure_env_modal_kernels() {
   return cudaSuccess;
 }
 
-int env_column_log_v(int n_to) { return column_log_v(31 - __builtin_clz((unsigned)n_to)); }
-int env_node_log_v(int n_to) { return regs::default_log_v(31 - __builtin_clz((unsigned)n_to)); }
-
-void row_twiddles(int n_to, int log_v, const std::vector<double2>& tw, std::vector<double2>& outer,
+void row_twiddles(int n_to, const std::vector<double2>& tw, std::vector<double2>& outer,
                   std::vector<double2>& inner) {
   // Row's V, T, M and G (the same for either type)
-  const int V = 1 << log_v, T = n_to / V, M = T, G = M / V;
+  const int log_v = regs::default_log_v(31 - __builtin_clz((unsigned)n_to)), V = 1 << log_v, T = n_to / V, M = T, G = M / V;
   auto root = [&](long q) {  // exp(-2 pi i q / 2n), q < 2n
     double2 w = tw[q & (n_to - 1)];
     if (q >= n_to) w = make_double2(-w.x, -w.y);
@@ -615,7 +616,7 @@ cudaError_t launch_env_inverse(const EnvModalArgsT<R>& a, const RamanArgs* raman
   return with_row<R>(a.log_n_to, [&](auto log) {
     constexpr int LOGN = decltype(log)::value;
     if constexpr (LOGN <= 13)
-      k_env_inverse<R, LOGN><<<a.n_cols + 2 * kernels, ColumnRow<double2, LOGN>::T, plane_smem<double2, LOGN>(), s>>>(
+      k_env_inverse<R, LOGN><<<a.n_cols + 2 * kernels, regs::Row<double2, LOGN>::T, plane_smem<double2, LOGN>(), s>>>(
           a, raman ? *raman : RamanArgs{}, table, 2 * kernels);
     return cudaGetLastError();
   });
@@ -649,7 +650,7 @@ cudaError_t launch_env_forward(const EnvModalArgsT<R>& a, cudaStream_t s) {
   }
   return with_row<R>(a.log_n_to, [&](auto log) {
     constexpr int LOGN = decltype(log)::value;
-    k_env_forward<R, LOGN><<<a.n_cols, ColumnRow<cplx<R>, LOGN>::T, plane_smem<cplx<R>, LOGN>(), s>>>(a);
+    k_env_forward<R, LOGN><<<a.n_cols, regs::Row<cplx<R>, LOGN>::T, plane_smem<cplx<R>, LOGN>(), s>>>(a);
     return cudaGetLastError();
   });
 }

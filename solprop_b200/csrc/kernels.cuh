@@ -275,15 +275,13 @@ struct EnvModalArgsT {
   double2* scratch;               // FP64 rows above kMaxEnvelopeRowF64: 1.5 n_to per row
   const double2* raman_spectrum;  // (raman_kernels, n_to + 1), or null without Raman
   const int* raman_scale;         // the mixed form: the powers of two inside raman_table
-  // the register transform of the nodes' rows (fft_regs.cuh): the spectra in its bin order,
+  // the register transform (fft_regs.cuh): the nodes' Raman spectra in its bin order,
   // (raman_kernels, 2 n_to), its two twiddle tables
   const cplx<R>* raman_table;
   const cplx<R>* outer_twiddles;
   const cplx<R>* inner_twiddles;
-  const double2* row_outer;       // the columns' transforms (rows of up to kMaxEnvelopeRowF64), FP64
+  const double2* row_outer;       // the same in FP64 (rows of up to kMaxEnvelopeRowF64)
   const double2* row_inner;
-  const cplx<R>* row_outer_r;     // ... and in the form's type
-  const cplx<R>* row_inner_r;
   const int* fine_to_coarse;      // (n_to): the coarse bin of a fine one, or -1
   int n_cols, n_omega, n_to, log_n_to, kerr, raman_mixture;
   int n_components;               // field components per node (1, or 2: rows x, y)
@@ -295,11 +293,8 @@ cudaError_t configure_env_modal_kernels();
 // nodes' a.raman_table
 template <class R>
 cudaError_t launch_env_inverse(const EnvModalArgsT<R>& a, const RamanArgs* raman, cplx<R>* table, cudaStream_t s);
-int env_column_log_v(int n_to);  // log2 of the points per thread of the columns' and the nodes' rows
-int env_node_log_v(int n_to);
-// the register transform's tables for V = 2^log_v points per thread, from exp(-2 pi i m / (2 n_to)),
-// m < n_to (fft_regs.cuh)
-void row_twiddles(int n_to, int log_v, const std::vector<double2>& tw, std::vector<double2>& outer,
+// the register transform's tables from exp(-2 pi i m / (2 n_to)), m < n_to (fft_regs.cuh)
+void row_twiddles(int n_to, const std::vector<double2>& tw, std::vector<double2>& outer,
                   std::vector<double2>& inner);
 template <class R>
 cudaError_t launch_env_nodes(const EnvModalArgsT<R>& a, int n_nodes, cudaStream_t s);
