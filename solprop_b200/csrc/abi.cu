@@ -466,7 +466,12 @@ static void fill_stage(sp_workspace* ws, int slot, double z0, double z1) {
   else s.pre_w[0] = 1.0;
 }
 
+// (one slot goes by value: no copy, and no wait for one before the slot is filled again)
 static void upload_stages(sp_workspace* ws, int count) {
+  if (count == 1 && !ws->borrowed) {
+    CUDA_CHECK(launch_put_stage(ws->h_stage[0], ws->stage.p, ws->stream));
+    return;
+  }
   CUDA_CHECK(cudaMemcpyAsync(ws->stage.p, ws->h_stage, count * sizeof(StageScalarsDev),
                              cudaMemcpyHostToDevice, ws->stream));
   release_host_tables(ws);
@@ -1492,15 +1497,15 @@ static void check_column(const double* h_norms, double* d_norms, cudaStream_t s)
 // step's two stage slots and tables from the pinned buffers, the predictor, the source at the
 // predicted field, the corrector with its reduction, the norms to the pinned host buffer.
 static void issue_attempt(sp_workspace* ws, const StepArgs& a) {
-  // the trial's table and the step's two stage slots, contiguous on both sides: one copy
-  CUDA_CHECK(cudaMemcpyAsync(ws->adams.p, ws->h_adams, sizeof(AdamsDev) + 2 * sizeof(StageScalarsDev),
-                             cudaMemcpyHostToDevice, ws->stream));
+  // the trial's table and the step's two stage slots, contiguous on both sides
+  static_assert((sizeof(AdamsDev) + 2 * sizeof(StageScalarsDev)) % 16 == 0, "fetched in 16-byte units");
+  CUDA_CHECK(launch_fetch_tables(ws->h_adams, ws->adams.p, sizeof(AdamsDev) + 2 * sizeof(StageScalarsDev),
+                                 ws->stream));
   { KernelTimer t(ws, SP_K_PREDICT); CUDA_CHECK(launch_adams_predict(a, ws->stream)); }
   eval_source(ws, ws->lab.p, 1, nullptr, ws->src.p, false, /*output=*/false);
   const OutputArgs oa = source_output_args(ws, 1, nullptr, ws->src.p, false);
-  { KernelTimer t(ws, SP_K_CORRECT); CUDA_CHECK(launch_adams_correct(a, &oa, ws->stream)); }
-  CUDA_CHECK(cudaMemcpyAsync(ws->h_norms, ws->norms.p, sizeof(double) * (kColumnStatus + 1),
-                             cudaMemcpyDeviceToHost, ws->stream));
+  KernelTimer t(ws, SP_K_CORRECT);
+  CUDA_CHECK(launch_adams_correct(a, &oa, ws->stream));
 }
 
 // One Adams attempt of a single run; returns accepted.  Without per-kernel timing the attempt
@@ -1510,6 +1515,7 @@ static bool adams_attempt(sp_session* S, double dz, double end, bool kink, bool 
   sp_workspace* ws = S->ws;
   Pending pd = prepare_attempt(S, dz, end, kink, fixed);
   StepArgs a = step_args_of(ws, ws->adams.p, ws->stage.p);
+  a.host_norms = ws->h_norms;
   if (ws->timing) {
     issue_attempt(ws, a);
   } else {

@@ -787,22 +787,26 @@ template <class R> constexpr int column_residency() { return sizeof(R) == 8 ? 2 
 
 template <class R>
 __global__ void __launch_bounds__(kThreads, column_residency<R>()) k_column(ColumnArgsT<R> a) {
+  await_previous_kernel();
   column_body(a);
 }
 
 template <class R>
 __global__ void __launch_bounds__(kThreads, column_residency<R>()) k_column_nodes(ColumnArgsT<R> a) {
+  await_previous_kernel();
   column_body<R, true>(a);
 }
 
 // a gas mixture's plasma channels, on either route
 template <class R>
 __global__ void __launch_bounds__(kThreads, column_residency<R>()) k_column_mix(ColumnArgsT<R> a) {
+  await_previous_kernel();
   column_body<R, false, true>(a);
 }
 
 template <class R>
 __global__ void __launch_bounds__(kThreads, column_residency<R>()) k_column_nodes_mix(ColumnArgsT<R> a) {
+  await_previous_kernel();
   column_body<R, true, true>(a);
 }
 
@@ -842,19 +846,15 @@ cudaError_t launch_column_b(const ColumnArgsT<R>* args, const int4* items, const
 template <class R>
 cudaError_t launch_column(const ColumnArgsT<R>& a, cudaStream_t stream) {
   if (a.plasma && a.n_channels > 1)
-    k_column_mix<R><<<a.n_blocks, kThreads, column_smem<R>(), stream>>>(a);
-  else
-    k_column<R><<<a.n_blocks, kThreads, column_smem<R>(), stream>>>(a);
-  return cudaGetLastError();
+    return launch_chained(k_column_mix<R>, a.n_blocks, kThreads, column_smem<R>(), 1, stream, a);
+  return launch_chained(k_column<R>, a.n_blocks, kThreads, column_smem<R>(), 1, stream, a);
 }
 
 template <class R>
 cudaError_t launch_column_nodes(const ColumnArgsT<R>& a, cudaStream_t stream) {
   if (a.plasma && a.n_channels > 1)
-    k_column_nodes_mix<R><<<a.n_blocks, kThreads, column_smem<R>(), stream>>>(a);
-  else
-    k_column_nodes<R><<<a.n_blocks, kThreads, column_smem<R>(), stream>>>(a);
-  return cudaGetLastError();
+    return launch_chained(k_column_nodes_mix<R>, a.n_blocks, kThreads, column_smem<R>(), 1, stream, a);
+  return launch_chained(k_column_nodes<R>, a.n_blocks, kThreads, column_smem<R>(), 1, stream, a);
 }
 
 template cudaError_t launch_column_nodes<double>(const ColumnArgsT<double>&, cudaStream_t);

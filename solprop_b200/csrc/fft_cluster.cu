@@ -137,6 +137,7 @@ __device__ __forceinline__ void inverse_cluster_body(const InverseArgsT<R>& a, i
 
 template <class R, int C>
 __global__ void __launch_bounds__(512) k_inverse_cluster(InverseArgsT<R> a) {
+  await_previous_kernel();
   inverse_cluster_body<C>(a, blockIdx.y);
 }
 
@@ -235,6 +236,7 @@ __device__ __forceinline__ void forward_cluster_body(const ForwardArgsT<R>& a, i
 
 template <class R, int C>
 __global__ void __launch_bounds__(512) k_forward_cluster(ForwardArgsT<R> a) {
+  await_previous_kernel();
   forward_cluster_body<C>(a, blockIdx.y);
 }
 
@@ -283,44 +285,39 @@ int single_transform_width(int n_to, size_t complex_bytes, bool forward) {
 }
 
 template <class R>
-static const void* single_inverse_kernel(int C) {
+static auto single_inverse_kernel(int C) -> void (*)(InverseArgsT<R>) {
   switch (C) {
-    case 2: return (const void*)k_inverse_cluster<R, 2>;
-    case 4: return (const void*)k_inverse_cluster<R, 4>;
-    case 8: return (const void*)k_inverse_cluster<R, 8>;
+    case 2: return k_inverse_cluster<R, 2>;
+    case 4: return k_inverse_cluster<R, 4>;
+    case 8: return k_inverse_cluster<R, 8>;
     default: return nullptr;
   }
 }
 template <class R>
-static const void* single_forward_kernel(int C) {
+static auto single_forward_kernel(int C) -> void (*)(ForwardArgsT<R>) {
   switch (C) {
-    case 2: return (const void*)k_forward_cluster<R, 2>;
-    case 4: return (const void*)k_forward_cluster<R, 4>;
-    case 8: return (const void*)k_forward_cluster<R, 8>;
+    case 2: return k_forward_cluster<R, 2>;
+    case 4: return k_forward_cluster<R, 4>;
+    case 8: return k_forward_cluster<R, 8>;
     default: return nullptr;
   }
 }
 
 template <class R>
 cudaError_t launch_inverse_cluster(const InverseArgsT<R>& a, int n_cols, int C, cudaStream_t stream) {
-  const void* kernel = single_inverse_kernel<R>(C);
+  const auto kernel = single_inverse_kernel<R>(C);
   if (!kernel) return cudaErrorInvalidValue;
   const int Mp = (a.n_to / 2) / C;
-  InverseArgsT<R> copy = a;
-  void* args[] = {&copy};
-  return launch_cluster(kernel, dim3(C, n_cols), Mp >= 512 ? 512 : Mp, (size_t)Mp * sizeof(cplx<R>), C,
-                        stream, args);
+  return launch_chained(kernel, dim3(C, n_cols), Mp >= 512 ? 512 : Mp, (size_t)Mp * sizeof(cplx<R>), C, stream, a);
 }
 
 template <class R>
 cudaError_t launch_forward_cluster(const ForwardArgsT<R>& a, int n_rows, int C, cudaStream_t stream) {
-  const void* kernel = single_forward_kernel<R>(C);
+  const auto kernel = single_forward_kernel<R>(C);
   if (!kernel) return cudaErrorInvalidValue;
   const int Mp = (a.n_to / 2) / C;
-  ForwardArgsT<R> copy = a;
-  void* args[] = {&copy};
-  return launch_cluster(kernel, dim3(C, n_rows), Mp >= 512 ? 512 : Mp, (size_t)2 * Mp * sizeof(cplx<R>), C,
-                        stream, args);
+  return launch_chained(kernel, dim3(C, n_rows), Mp >= 512 ? 512 : Mp, (size_t)2 * Mp * sizeof(cplx<R>), C, stream,
+                        a);
 }
 
 template <class R>
@@ -382,8 +379,8 @@ SP_CLUSTER_INSTANCES(float)
 cudaError_t configure_cluster_fft() {
   // single-run and batched kernels of every width: rows of up to kClusterSmem per CTA
   for (int C : {2, 4, 8}) {
-    for (const void* k : {single_inverse_kernel<double>(C), single_forward_kernel<double>(C),
-                          single_inverse_kernel<float>(C), single_forward_kernel<float>(C),
+    for (const void* k : {(const void*)single_inverse_kernel<double>(C), (const void*)single_forward_kernel<double>(C),
+                          (const void*)single_inverse_kernel<float>(C), (const void*)single_forward_kernel<float>(C),
                           inverse_cluster_kernel<double>(C), forward_cluster_kernel<double>(C),
                           inverse_cluster_kernel<float>(C), forward_cluster_kernel<float>(C)}) {
       cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterSmem);

@@ -388,10 +388,16 @@ struct StepArgs {
   double* partials;           // (kMaxOrders + 2, kNormBlocks)
   double* norms;              // (kMaxOrders + 2)
   int n_blocks;               // blocks of the grid-stride loops (<= kNormBlocks)
+  double* host_norms;         // single run: pinned host memory the last block writes the norms and the
+                              // column's status to as well; null: the host copies them
   unsigned* norm_arrivals;    // single run: the corrector's block count (its last block
                               // reduces the partials); null: a separate reduction launch
 };
 
+// one stage's scalars, by value; a table of pinned host memory (16-byte aligned, whole 16-byte
+// units) read by the device: a short kernel in the chain in place of a copy
+cudaError_t launch_put_stage(const StageScalarsDev& value, StageScalarsDev* dst, cudaStream_t stream);
+cudaError_t launch_fetch_tables(const void* pinned, void* dst, size_t bytes, cudaStream_t stream);
 cudaError_t launch_adams_predict(const StepArgs& a, cudaStream_t stream);
 // with an output record (non-null), the corrector forms the source row itself: the stage
 // output pass of the source evaluation before it, fused

@@ -83,6 +83,7 @@ __device__ __forceinline__ void inverse_field_body(const InverseArgsT<R>& a, int
 
 template <class R>
 __global__ void __launch_bounds__(kRowThreads) k_inverse_field(InverseArgsT<R> a) {
+  await_previous_kernel();
   inverse_field_body(a, blockIdx.x);
 }
 
@@ -174,6 +175,7 @@ __device__ __forceinline__ void forward_field_body(const ForwardArgsT<R>& a, int
 
 template <class R>
 __global__ void __launch_bounds__(kRowThreads) k_forward_field(ForwardArgsT<R> a) {
+  await_previous_kernel();
   forward_field_body(a, blockIdx.x);
 }
 
@@ -192,7 +194,10 @@ __device__ __forceinline__ void stage_output_any(const OutputArgs& a, int block)
   if (idx < a.n_cols * a.n_omega) a.out[idx] = stage_output_value(a, idx);
 }
 
-__global__ void k_stage_output(OutputArgs a) { stage_output_any(a, blockIdx.x); }
+__global__ void k_stage_output(OutputArgs a) {
+  await_previous_kernel();
+  stage_output_any(a, blockIdx.x);
+}
 
 // batched: items[blockIdx.x] = (run, block of 256 elements)
 __global__ void k_stage_output_b(const OutputArgs* args, const int2* items, const int* flags) {
@@ -216,8 +221,7 @@ cudaError_t launch_inverse(const InverseArgsT<R>& a, int n_cols, cudaStream_t st
   const int C = single_transform_width(a.n_to, sizeof(cplx<R>), false);
   if (C > 1) return launch_inverse_cluster(a, n_cols, C, stream);
   const int M = a.n_to >> 1;
-  k_inverse_field<R><<<n_cols, threads_for<R>(M), row_smem<R>(M), stream>>>(a);
-  return cudaGetLastError();
+  return launch_chained(k_inverse_field<R>, n_cols, threads_for<R>(M), row_smem<R>(M), 1, stream, a);
 }
 
 template <class R>
@@ -225,8 +229,7 @@ cudaError_t launch_forward(const ForwardArgsT<R>& a, int n_rows, cudaStream_t st
   const int C = single_transform_width(a.n_to, sizeof(cplx<R>), true);
   if (C > 1) return launch_forward_cluster(a, n_rows, C, stream);
   const int M = a.n_to >> 1;
-  k_forward_field<R><<<n_rows, threads_for<R>(M), row_smem<R>(M), stream>>>(a);
-  return cudaGetLastError();
+  return launch_chained(k_forward_field<R>, n_rows, threads_for<R>(M), row_smem<R>(M), 1, stream, a);
 }
 
 template cudaError_t launch_inverse<double>(const InverseArgsT<double>&, int, cudaStream_t);
@@ -236,8 +239,7 @@ template cudaError_t launch_forward<float>(const ForwardArgsT<float>&, int, cuda
 
 cudaError_t launch_output(const OutputArgs& a, cudaStream_t stream) {
   const int total = a.n_cols * a.n_omega;
-  k_stage_output<<<(total + 255) / 256, 256, 0, stream>>>(a);
-  return cudaGetLastError();
+  return launch_chained(k_stage_output, (total + 255) / 256, 256, 0, 1, stream, a);
 }
 
 cudaError_t configure_source_kernels() {

@@ -63,6 +63,36 @@ template <> __host__ __device__ __forceinline__ float2 to_c<float2>(double2 v) {
 __host__ __device__ __forceinline__ double2 to_d2(double2 v) { return v; }
 __host__ __device__ __forceinline__ double2 to_d2(float2 v) { return make_double2(v.x, v.y); }
 
+// ---- a single run's chain of short kernels: each is launched while the one before it runs
+// (programmatic dependent launch) and waits here, before its first access to global memory,
+// for that one's end; and it lets the next be launched at once.  Every kernel of the chain
+// waits, so each sees the writes of all before it.  A kernel launched in the ordinary way
+// passes straight through.  It saves a launch's latency per kernel, about 1 us of 5.
+__device__ __forceinline__ void await_previous_kernel() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// launches a kernel that begins with await_previous_kernel, in clusters of `cluster` CTAs along x
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t shm, int cluster,
+                                  cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = shm;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // exp of a complex number
 __device__ __forceinline__ double2 cexp(double2 z) {
   double e = exp(z.x), s, c;

@@ -187,9 +187,15 @@ __device__ __forceinline__ void reduce_if_last(const StepArgs& a, int nq) {
     double x = 0.0;
     for (int b = lane; b < a.n_blocks; b += 32) x += __ldcg(a.partials + q * kNormBlocks + b);
     for (int d = 16; d > 0; d >>= 1) x += __shfl_down_sync(0xffffffffu, x, d);
-    if (lane == 0) a.norms[q] = x;
+    if (lane == 0) {
+      a.norms[q] = x;
+      if (a.host_norms) a.host_norms[q] = x;
+    }
   }
-  if (threadIdx.x == 0) *a.norm_arrivals = 0u;
+  if (threadIdx.x == 0) {
+    *a.norm_arrivals = 0u;
+    if (a.host_norms) a.host_norms[kColumnStatus] = __ldcg(a.norms + kColumnStatus);
+  }
 }
 
 // The trial's coefficient table, copied into shared memory once per block.  Every thread
@@ -474,9 +480,11 @@ __device__ __forceinline__ void adams_start_body(const StepArgs& a, int write_ra
 // bound by HBM: the register budget is capped so that more warps keep loads in flight.
 constexpr int kStepThreads = 128;
 __global__ void __launch_bounds__(2 * kStepThreads) k_adams_predict(StepArgs a) {
+  await_previous_kernel();
   adams_predict_body<true>(a, blockIdx.x);
 }
 __global__ void __launch_bounds__(2 * kStepThreads) k_adams_correct(StepArgs a, const __grid_constant__ OutputArgs o) {
+  await_previous_kernel();
   adams_correct_body<true>(a, blockIdx.x, o.out ? &o : nullptr);
   if (a.norm_arrivals) reduce_if_last(a, kMaxOrders + 1);
 }
@@ -509,12 +517,34 @@ __global__ void k_adams_start_b(const StepArgs* args, const int2* items, const i
   adams_start_body(a, a.states != nullptr, it.y);
 }
 
+// What bounds these two: a copy through the copy engine and the hand-over to and from it cost a
+// chain of 5 us kernels a few microseconds; a kernel's launch overlaps its neighbours'.
+static_assert(sizeof(StageScalarsDev) % 8 == 0, "copied in 8-byte words");
+__global__ void k_put_stage(const __grid_constant__ StageScalarsDev value, StageScalarsDev* dst) {
+  await_previous_kernel();
+  const double* from = reinterpret_cast<const double*>(&value);
+  for (int i = threadIdx.x; i < (int)(sizeof(StageScalarsDev) / 8); i += blockDim.x)
+    reinterpret_cast<double*>(dst)[i] = from[i];
+}
+__global__ void k_fetch_tables(const uint4* pinned, uint4* dst, int count) {
+  await_previous_kernel();
+  for (int i = threadIdx.x; i < count; i += blockDim.x) dst[i] = __ldcv(pinned + i);
+}
+cudaError_t launch_put_stage(const StageScalarsDev& value, StageScalarsDev* dst, cudaStream_t s) {
+  return launch_chained(k_put_stage, 1, 256, 0, 1, s, value, dst);
+}
+cudaError_t launch_fetch_tables(const void* pinned, void* dst, size_t bytes, cudaStream_t s) {
+  return launch_chained(k_fetch_tables, 1, 512, 0, 1, s, static_cast<const uint4*>(pinned), static_cast<uint4*>(dst),
+                        (int)(bytes / 16));
+}
+
 cudaError_t launch_adams_predict(const StepArgs& a, cudaStream_t s) {
-  k_adams_predict<<<a.n_blocks, 2 * kStepThreads, 0, s>>>(a);
-  return cudaGetLastError();
+  return launch_chained(k_adams_predict, a.n_blocks, 2 * kStepThreads, 0, 1, s, a);
 }
 cudaError_t launch_adams_correct(const StepArgs& a, const OutputArgs* output, cudaStream_t s) {
-  k_adams_correct<<<a.n_blocks, 2 * kStepThreads, 0, s>>>(a, output ? *output : OutputArgs{});
+  const cudaError_t e = launch_chained(k_adams_correct, a.n_blocks, 2 * kStepThreads, 0, 1, s, a,
+                                       output ? *output : OutputArgs{});
+  if (e != cudaSuccess) return e;
   if (!a.norm_arrivals) k_reduce<<<kMaxOrders + 1, 32, 0, s>>>(a.partials, a.norms, kMaxOrders + 1, a.n_blocks);
   return cudaGetLastError();
 }
