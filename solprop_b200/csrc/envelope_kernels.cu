@@ -46,6 +46,7 @@ constexpr size_t envelope_smem() {
 template <int LOGN>
 __global__ void __cluster_dims__(kRanks, 1, 1) __launch_bounds__(EnvelopeRow<LOGN>::T)
     k_envelope_source(EnvelopeArgs a) {
+  await_previous_kernel();
   using Row = EnvelopeRow<LOGN>;
   constexpr int n = Row::N, T = Row::T, V = Row::V;
   extern __shared__ __align__(16) unsigned char env_raw[];
@@ -164,8 +165,7 @@ static cudaError_t with_envelope_row(int log_n, F&& f) {
 cudaError_t launch_envelope(const EnvelopeArgs& a, cudaStream_t stream) {
   return with_envelope_row(a.log_n_to, [&](auto log) {
     constexpr int LOGN = decltype(log)::value;
-    k_envelope_source<LOGN><<<kRanks, EnvelopeRow<LOGN>::T, envelope_smem<LOGN>(), stream>>>(a);
-    return cudaGetLastError();
+    return launch_chained(k_envelope_source<LOGN>, kRanks, EnvelopeRow<LOGN>::T, envelope_smem<LOGN>(), 1, stream, a);
   });
 }
 

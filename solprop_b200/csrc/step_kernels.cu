@@ -158,6 +158,7 @@ __device__ __forceinline__ void reduce_body(const double* partials, double* out,
 }
 
 __global__ void k_reduce(const double* partials, double* out, int nq, int nb) {
+  await_previous_kernel();
   if ((int)blockIdx.x >= nq) return;
   reduce_body(partials, out, blockIdx.x, nb);
 }
@@ -580,6 +581,7 @@ struct RkCoeffs {
 };
 
 __global__ void __launch_bounds__(256) k_rk_stage_input(RkArgs a, RkCoeffs c) {
+  await_previous_kernel();
   const StageScalarsDev& st = *a.stage;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
     const double2 x = combine_terms(st.phi_w, st.n_phi, a.phi_terms, a.n, i);
@@ -608,6 +610,7 @@ struct RkFinish {
 };
 
 __global__ void __launch_bounds__(256) k_rk_finish(RkArgs a, RkFinish f) {
+  await_previous_kernel();
   const StageScalarsDev& st = *a.stage;
   double v[3] = {0.0, 0.0, 0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
@@ -646,8 +649,7 @@ cudaError_t launch_rk_stage_input(const RkArgs& a, int stage, const double* coef
   for (int j = 0; j < stage && j < 8; ++j) c.a[j] = coeffs[j];
   c.stage = stage;
   c.dz = dz;
-  k_rk_stage_input<<<kNormBlocks, 256, 0, s>>>(a, c);
-  return cudaGetLastError();
+  return launch_chained(k_rk_stage_input, kNormBlocks, 256, 0, 1, s, a, c);
 }
 
 cudaError_t launch_rk_finish(const RkArgs& a, const double* b, const double* e, double dz,
@@ -658,9 +660,9 @@ cudaError_t launch_rk_finish(const RkArgs& a, const double* b, const double* e, 
     f.e[j] = e[j];
   }
   f.dz = dz;
-  k_rk_finish<<<kNormBlocks, 256, 0, s>>>(a, f);
-  k_reduce<<<3, 32, 0, s>>>(a.partials, a.norms, 3, kNormBlocks);
-  return cudaGetLastError();
+  const cudaError_t status = launch_chained(k_rk_finish, kNormBlocks, 256, 0, 1, s, a, f);
+  if (status != cudaSuccess) return status;
+  return launch_chained(k_reduce, 3, 32, 0, 1, s, a.partials, a.norms, 3, kNormBlocks);
 }
 
 cudaError_t launch_mask_copy(double2* dst, const double2* src, const unsigned char* active, int n,
