@@ -164,7 +164,17 @@ __device__ __forceinline__ void forward_cluster_body(const ForwardArgsT<R>& a, i
   const int log_mp = a.log_m - __ffs(C) + 1;
   Cx* zb = sc + Mp;  // Z for this CTA's k1 slice: [k2][k1 - r slice]
   const int slice = Mp / C;
-  // z[C n2 + r] = x[2(C n2 + r)] + i x[2(C n2 + r) + 1]
+  // z[m] = x[2m] + i x[2m + 1] belongs to CTA m mod C.  Each CTA reads a contiguous slice of the
+  // row and hands its samples out through distributed shared memory: read where they belong,
+  // every C-th sample, a warp's load would touch 32 sectors for 16 bytes of each, over every
+  // node group (five modes and groups, FP32: 32.1 -> 28.6 us an evaluation).  A row of one group
+  // is read where it belongs: there the cluster's two barriers cost more (one mode: +2 %).
+  const bool hand_out = row < a.n_partial_rows && a.n_groups > 1;  // uniform over the cluster
+  Cx* home = sc;  // of every sample this thread reads
+  if (hand_out) {
+    home = cluster.map_shared_rank(sc, (unsigned)threadIdx.x % C);
+    cluster.sync();  // every CTA of the cluster runs
+  }
   if (row < a.n_partial_rows) {
     // a projected stream: the node groups' partial rows summed in group order, eight
     // groups' loads issued before their sums
@@ -172,8 +182,8 @@ __device__ __forceinline__ void forward_cluster_body(const ForwardArgsT<R>& a, i
     const Cx* rows = reinterpret_cast<const Cx*>(a.partials + (size_t)row * a.n_to);
     const size_t group_stride = (size_t)a.n_partial_rows * a.n_to / 2;  // in complex samples
 #pragma unroll 2
-    for (int n2 = threadIdx.x; n2 < Mp; n2 += blockDim.x) {
-      const int m = C * n2 + r;
+    for (int v = threadIdx.x; v < Mp; v += blockDim.x) {
+      const int m = hand_out ? r * Mp + v : C * v + r;
       Cx acc;
       acc.x = R(0);
       acc.y = R(0);
@@ -188,14 +198,15 @@ __device__ __forceinline__ void forward_cluster_body(const ForwardArgsT<R>& a, i
           acc = cadd(acc, x[g]);
         }
       }
-      sc[row_slot<Cx>(n2)] = acc;
+      home[row_slot<Cx>(m / C)] = acc;
     }
   } else {
     const double2* x = reinterpret_cast<const double2*>(a.streams + (size_t)row * a.n_to);
 #pragma unroll 4
     for (int n2 = threadIdx.x; n2 < Mp; n2 += blockDim.x) sc[row_slot<Cx>(n2)] = to_c<Cx>(x[C * n2 + r]);
   }
-  __syncthreads();
+  if (hand_out) cluster.sync();
+  else __syncthreads();
   fft_dif_swizzled</*kInv=*/false>(sc, log_mp, a.twiddles, a.log_n_to);
   cluster.sync();
   for (int kk = threadIdx.x; kk < slice; kk += blockDim.x) {
