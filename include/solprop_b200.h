@@ -454,6 +454,21 @@ sp_status sp_mlp_layer_backward(const float* dA, const float* pre, int M, int N,
                                 int rows_pad, float* db, void* stream);
 sp_status sp_mlp_first_layer_backward(const float* dA, const float* pre, const float* x, int ldx, int M,
                                       int N, int K, float* dW, float* db, void* stream);
+/* The launches of a training pass over `layers` (at most SP_MLP_MAX_LAYERS) linear layers, W[i] (n[i],
+ * k[i]) with k[i + 1] = n[i], on the tcgen05 products (their rules on n and k; k[0] is free): forward
+ * writes pre[i] (FP32) and act[i] (BF16) of the hidden layers and out; backward reads them (pre[i]
+ * NULL: no GELU) and writes every dW and db.  scratch: sp_mlp_training_scratch bytes of device memory. */
+#define SP_MLP_MAX_LAYERS 16
+size_t sp_mlp_training_scratch(int layers, int M, const int* n, const int* k);
+sp_status sp_mlp_training_forward(int layers, int M, const int* n, const int* k, const float* const* W,
+                                  const float* const* bias, const float* x, int ldx, float* const* pre,
+                                  void* const* act, float* out, void* scratch, size_t scratch_bytes,
+                                  int* status, void* stream);
+sp_status sp_mlp_training_backward(int layers, int M, const int* n, const int* k, const float* const* W,
+                                   const float* x, int ldx, const float* const* pre,
+                                   const void* const* act, const float* dy, float* const* dW,
+                                   float* const* db, void* scratch, size_t scratch_bytes, int* status,
+                                   void* stream);
 /* sp_mlp_adam for up to 16 parameters, sp_mlp_to_bf16 / sp_mlp_transpose_bf16 for up to 8 matrices, in
  * one launch: copy[q] (rows, cols_out) and transpose[q] (cols, rows_pad), either NULL. */
 sp_status sp_mlp_adam_batch(int count, float* const* w, const float* const* grad, float* const* m1,

@@ -176,6 +176,15 @@ SIGNATURES = {
                              C.c_void_p, C.c_void_p]),
     "sp_mlp_adam": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_float,
                               C.c_float, C.c_float, C.c_float, C.c_int, C.c_void_p]),
+    "sp_mlp_training_scratch": (C.c_size_t, [C.c_int, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
+    "sp_mlp_training_forward": (C.c_int, [C.c_int, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int),
+                                          C.POINTER(C.c_void_p), C.POINTER(C.c_void_p), C.c_void_p, C.c_int,
+                                          C.POINTER(C.c_void_p), C.POINTER(C.c_void_p), C.c_void_p, C.c_void_p,
+                                          C.c_size_t, C.c_void_p, C.c_void_p]),
+    "sp_mlp_training_backward": (C.c_int, [C.c_int, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int),
+                                           C.POINTER(C.c_void_p), C.c_void_p, C.c_int, C.POINTER(C.c_void_p),
+                                           C.POINTER(C.c_void_p), C.c_void_p, C.POINTER(C.c_void_p),
+                                           C.POINTER(C.c_void_p), C.c_void_p, C.c_size_t, C.c_void_p, C.c_void_p]),
     "sp_mlp_layer_backward": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_void_p,
                                         C.c_int, C.c_void_p, C.c_void_p]),
     "sp_mlp_first_layer_backward": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int,

@@ -432,6 +432,56 @@ bool make_map(CUtensorMap* map, const void* base, int rows, int cols, int ld, in
 }  // namespace
 }  // namespace sp
 
+namespace {
+struct Carve {  // 256-byte aligned pieces of the caller's scratch; counts alone when base is null
+  char* base;
+  size_t used = 0;
+  template <class T>
+  T* take(size_t count) {
+    T* p = base ? reinterpret_cast<T*>(base + used) : nullptr;
+    used += (count * sizeof(T) + 255) / 256 * 256;
+    return p;
+  }
+};
+int pad64(int v) { return (v + 63) / 64 * 64; }
+bool training_sizes(int layers, int M, const int* n, const int* k) {
+  if (layers < 1 || layers > SP_MLP_MAX_LAYERS || M < 1 || !n || !k) return false;
+  for (int i = 0; i < layers; ++i)
+    if (n[i] < 1 || k[i] < 1 || (i && k[i] != n[i - 1])) return false;
+  return true;
+}
+struct ForwardScratch {
+  void* a;
+  void* w[SP_MLP_MAX_LAYERS];
+  size_t bytes;
+  ForwardScratch(void* base, int layers, int M, const int* n, const int* k) {
+    Carve c{static_cast<char*>(base)};
+    a = c.take<__nv_bfloat16>((size_t)M * pad64(k[0]));
+    for (int i = 0; i < layers; ++i) w[i] = c.take<__nv_bfloat16>((size_t)n[i] * pad64(k[i]));
+    bytes = c.used;
+  }
+};
+struct BackwardScratch {
+  void *wt[SP_MLP_MAX_LAYERS], *at[SP_MLP_MAX_LAYERS], *dzt[SP_MLP_MAX_LAYERS], *dz;
+  float* g[2];
+  size_t bytes;
+  BackwardScratch(void* base, int layers, int M, const int* n, const int* k) {
+    Carve c{static_cast<char*>(base)};
+    const int rows = pad64(M);
+    int widest = n[0];
+    for (int i = 1; i < layers; ++i) {
+      wt[i] = c.take<__nv_bfloat16>((size_t)k[i] * n[i]);
+      at[i] = c.take<__nv_bfloat16>((size_t)k[i] * rows);
+      dzt[i] = c.take<__nv_bfloat16>((size_t)n[i] * rows);
+      if (n[i] > widest) widest = n[i];
+    }
+    dz = c.take<__nv_bfloat16>((size_t)M * widest);
+    for (float*& b : g) b = c.take<float>((size_t)M * widest);
+    bytes = c.used;
+  }
+};
+}  // namespace
+
 extern "C" {
 
 sp_status sp_mlp_gemm_tc_batch(int count, const void* const* A, int lda, const void* const* W, int ldw,
@@ -539,6 +589,102 @@ sp_status sp_mlp_to_bf16(const float* src, int ld_src, int rows, int cols, void*
   sp::k_to_bf16<<<blocks, 256, 0, (cudaStream_t)stream>>>(src, ld_src, rows, cols,
                                                           static_cast<__nv_bfloat16*>(dst), ld_dst, cols_out);
   return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ERR_CUDA;
+}
+
+// ---- a training pass's launches from one call: from Python each of two dozen launches and the
+// buffers between them cost the host more (345 us a step at a batch of 256) than the device
+size_t sp_mlp_training_scratch(int layers, int M, const int* n, const int* k) {
+  if (!training_sizes(layers, M, n, k)) return 0;
+  const size_t f = ForwardScratch(nullptr, layers, M, n, k).bytes, b = BackwardScratch(nullptr, layers, M, n, k).bytes;
+  return f > b ? f : b;
+}
+
+sp_status sp_mlp_training_forward(int layers, int M, const int* n, const int* k, const float* const* W,
+                                  const float* const* bias, const float* x, int ldx, float* const* pre,
+                                  void* const* act, float* out, void* scratch, size_t scratch_bytes, int* status,
+                                  void* stream) {
+  if (!training_sizes(layers, M, n, k) || !W || !bias || !x || !pre || !act || !out || !scratch || !status)
+    return SP_ERR_ARGUMENT;
+  const ForwardScratch s(scratch, layers, M, n, k);
+  if (s.bytes > scratch_bytes) return SP_ERR_ARGUMENT;
+  const void* src[SP_MLP_MAX_LAYERS + 1] = {x};
+  void* copy[SP_MLP_MAX_LAYERS + 1] = {s.a};
+  void* none[SP_MLP_MAX_LAYERS + 1] = {};
+  int rows[SP_MLP_MAX_LAYERS + 1] = {M}, cols[SP_MLP_MAX_LAYERS + 1] = {k[0]}, ld[SP_MLP_MAX_LAYERS + 1] = {ldx};
+  int wide[SP_MLP_MAX_LAYERS + 1] = {pad64(k[0])}, zero[SP_MLP_MAX_LAYERS + 1] = {};
+  for (int i = 0; i < layers; ++i) {
+    src[i + 1] = W[i];
+    copy[i + 1] = s.w[i];
+    rows[i + 1] = n[i];
+    cols[i + 1] = ld[i + 1] = k[i];
+    wide[i + 1] = pad64(k[i]);
+  }
+  for (int q = 0; q <= layers; q += sp::kMaxConversions) {
+    const int count = layers + 1 - q < sp::kMaxConversions ? layers + 1 - q : sp::kMaxConversions;
+    const sp_status e = sp_mlp_convert_batch(count, 0, src + q, rows + q, cols + q, ld + q, copy + q, wide + q,
+                                             none + q, zero + q, stream);
+    if (e != SP_OK) return e;
+  }
+  for (int i = 0; i < layers; ++i) {
+    const bool last = i == layers - 1;
+    const sp_status e = sp_mlp_gemm_tc(i ? act[i - 1] : s.a, i ? k[i] : pad64(k[0]), s.w[i], pad64(k[i]),
+                                       last ? out : pre[i], n[i], last ? nullptr : act[i], last ? 0 : n[i], M, n[i],
+                                       pad64(k[i]), bias[i], last ? 1 : 3, status, stream);
+    if (e != SP_OK) return e;
+  }
+  return SP_OK;
+}
+
+sp_status sp_mlp_training_backward(int layers, int M, const int* n, const int* k, const float* const* W,
+                                   const float* x, int ldx, const float* const* pre, const void* const* act,
+                                   const float* dy, float* const* dW, float* const* db, void* scratch,
+                                   size_t scratch_bytes, int* status, void* stream) {
+  if (!training_sizes(layers, M, n, k) || !W || !x || !pre || !act || !dy || !dW || !db || !scratch || !status)
+    return SP_ERR_ARGUMENT;
+  const BackwardScratch s(scratch, layers, M, n, k);
+  if (s.bytes > scratch_bytes) return SP_ERR_ARGUMENT;
+  const int rows_pad = pad64(M);
+  // the transposes: weights (n, k) -> (k, n), activations (M, k) -> (k, rows_pad)
+  int batch[SP_MLP_MAX_LAYERS], pads[SP_MLP_MAX_LAYERS], zero[SP_MLP_MAX_LAYERS] = {};
+  void* none[SP_MLP_MAX_LAYERS] = {};
+  for (int i = 0; i < layers; ++i) {
+    batch[i] = M;
+    pads[i] = rows_pad;
+  }
+  for (int i = 1; i < layers; i += sp::kMaxConversions) {
+    const int count = layers - i < sp::kMaxConversions ? layers - i : sp::kMaxConversions;
+    sp_status e = sp_mlp_convert_batch(count, 0, reinterpret_cast<const void* const*>(W + i), n + i, k + i, k + i, none,
+                                       zero, s.wt + i, n + i, stream);
+    if (e == SP_OK)
+      e = sp_mlp_convert_batch(count, 1, act + i - 1, batch, k + i, k + i, none, zero, s.at + i, pads, stream);
+    if (e != SP_OK) return e;
+  }
+  const float* g = dy;
+  for (int i = layers - 1; i > 0; --i) {
+    float* next = s.g[i & 1];
+    sp_status e = sp_mlp_layer_backward(g, pre[i], M, n[i], s.dz, s.dzt[i], rows_pad, db[i], stream);
+    if (e == SP_OK)
+      e = sp_mlp_gemm_tc(s.dz, n[i], s.wt[i], n[i], next, k[i], nullptr, 0, M, k[i], n[i], nullptr, 0, status, stream);
+    if (e != SP_OK) return e;
+    g = next;
+  }
+  // the weight gradients, neighbouring layers of one shape in one launch
+  for (int i = 1; i < layers;) {
+    int count = 1;
+    while (i + count < layers && count < sp::kMaxProducts && n[i + count] == n[i] && k[i + count] == k[i]) ++count;
+    const sp_status e = sp_mlp_gemm_tc_batch(count, s.dzt + i, rows_pad, s.at + i, rows_pad, dW + i, k[i], nullptr, 0,
+                                             n[i], k[i], rows_pad, nullptr, 0, status, stream);
+    if (e != SP_OK) return e;
+    i += count;
+  }
+  if (k[0] <= 8) return sp_mlp_first_layer_backward(g, pre[0], x, ldx, M, n[0], k[0], dW[0], db[0], stream);
+  // a wider first layer: the FP32-accumulating product (g is this call's own unless one layer is all)
+  float* dz = layers > 1 ? const_cast<float*>(g) : s.g[0];
+  sp_status e = SP_OK;
+  if (pre[0]) e = sp_mlp_gelu_backward(g, pre[0], dz, (size_t)M * n[0], stream);
+  const float* z = pre[0] ? dz : g;
+  if (e == SP_OK) e = sp_mlp_gemm(z, n[0], 1, x, ldx, 0, dW[0], k[0], n[0], k[0], M, nullptr, 0, nullptr, stream);
+  return e == SP_OK ? sp_mlp_bias_grad(z, M, n[0], db[0], stream) : e;
 }
 
 }  // extern "C"

@@ -272,21 +272,27 @@ class Perceptron:
         activations in BF16 (epilogue 3).  Returns the output, the cache and the status."""
         import torch
 
-        inputs = [x, *self.weights]
-        (a, *w16s), _ = convert_batch(inputs, [_pad64(t.shape[1]) for t in inputs])
-        cache = []
-        last = len(self.weights) - 1
-        for i, (w, w16, b) in enumerate(zip(self.weights, w16s, self.biases)):
-            if i == last:
-                out = torch.empty((a.shape[0], w.shape[0]), dtype=torch.float32, device=self.device)
-                status = gemm_tc(a, w16, out=out, bias=b, epilogue=1, status=status)
-                cache.append((x if i == 0 else a, None))
-                return out, cache, status
-            pre = torch.empty((a.shape[0], w.shape[0]), dtype=torch.float32, device=self.device)
-            nxt = torch.empty((a.shape[0], w.shape[0]), dtype=torch.bfloat16, device=self.device)
-            status = gemm_tc(a, w16, out=pre, out16=nxt, bias=b, epilogue=3, status=status)
-            cache.append((x if i == 0 else a, pre if keep else None))
-            a = nxt
+        m, hidden = x.shape[0], self.weights[:-1]
+        pre = [torch.empty((m, w.shape[0]), dtype=torch.float32, device=self.device) for w in hidden]
+        act = [torch.empty((m, w.shape[0]), dtype=torch.bfloat16, device=self.device) for w in hidden]
+        out = torch.empty((m, self.weights[-1].shape[0]), dtype=torch.float32, device=self.device)
+        if status is None:
+            status = torch.zeros(1, dtype=torch.int32, device=x.device)
+        sizes, scratch = self._training_pass(m)
+        _check(_bind().sp_mlp_training_forward(
+            *sizes, _pointers(self.weights), _pointers(self.biases), _ptr(x), x.stride(0), _pointers(pre),
+            _pointers(act), _ptr(out), _ptr(scratch), scratch.numel(), _ptr(status), None))
+        kept = pre if keep else [None] * len(pre)
+        return out, list(zip([x, *act], [*kept, None])), status
+
+    def _training_pass(self, m: int):
+        """The native training passes' sizes and their scratch for a batch of m."""
+        import torch
+
+        n = (C.c_int * len(self.weights))(*[w.shape[0] for w in self.weights])
+        k = (C.c_int * len(self.weights))(*[w.shape[1] for w in self.weights])
+        size = _bind().sp_mlp_training_scratch(len(n), m, n, k)
+        return (len(n), m, n, k), torch.empty(size, dtype=torch.uint8, device=self.device)
 
     def gradients_tc(self, cache, dy, status=None):
         """dW, db of every layer from dL/dy on the tcgen05 products: the weight gradient
@@ -298,44 +304,15 @@ class Perceptron:
         launch.  Returns (grads, status)."""
         import torch
 
-        lib = _bind()
         grads = [torch.empty_like(p) for p in self.params]
         if status is None:
             status = torch.zeros(1, dtype=torch.int32, device=dy.device)
-        last = len(self.weights) - 1
-        m, rows = dy.shape[0], _pad64(dy.shape[0])
-        upper = range(1, last + 1)
-        w16t = convert_batch([self.weights[i] for i in upper], None, [self.weights[i].shape[0] for i in upper])[1]
-        a16t = convert_batch([cache[i][0] for i in upper], None, [rows] * last)[1]
-        g = dy
-        dz16t = [None] * (last + 1)
-        for i in range(last, 0, -1):
-            pre = cache[i][1]
-            n, k = self.weights[i].shape
-            dz16 = torch.empty((m, n), dtype=torch.bfloat16, device=self.device)
-            dz16t[i] = torch.empty((n, rows), dtype=torch.bfloat16, device=self.device)
-            _check(lib.sp_mlp_layer_backward(_ptr(g), None if pre is None else _ptr(pre), m, n, _ptr(dz16),
-                                             _ptr(dz16t[i]), rows, _ptr(grads[2 * i + 1]), None))
-            g = torch.empty((m, k), dtype=torch.float32, device=self.device)
-            status = gemm_tc(dz16, w16t[i - 1], out=g, status=status)
-        # the weight gradients, the layers of one shape together
-        shapes = {}
-        for i in upper:
-            shapes.setdefault(self.weights[i].shape, []).append(i)
-        for alike in shapes.values():
-            for layers in (alike[s:s + 8] for s in range(0, len(alike), 8)):
-                status = gemm_tc_batch([dz16t[i] for i in layers], [a16t[i - 1] for i in layers],
-                                       outs=[grads[2 * i] for i in layers], status=status)
-        x, pre = cache[0]
-        n, k = self.weights[0].shape
-        if k <= 8:
-            _check(lib.sp_mlp_first_layer_backward(_ptr(g), None if pre is None else _ptr(pre), _ptr(x), x.stride(0),
-                                                   m, n, k, _ptr(grads[0]), _ptr(grads[1]), None))
-        else:
-            if pre is not None:
-                _check(lib.sp_mlp_gelu_backward(_ptr(g), _ptr(pre), _ptr(g), g.numel(), None))
-            gemm(g, x, grads[0], trans_a=True)
-            _check(lib.sp_mlp_bias_grad(_ptr(g), m, n, _ptr(grads[1]), None))
+        x = cache[0][0]
+        sizes, scratch = self._training_pass(dy.shape[0])
+        _check(_bind().sp_mlp_training_backward(
+            *sizes, _pointers(self.weights), _ptr(x), x.stride(0), _pointers([pre for _, pre in cache]),
+            _pointers([a for a, _ in cache[1:]]), _ptr(dy), _pointers(grads[::2]), _pointers(grads[1::2]),
+            _ptr(scratch), scratch.numel(), _ptr(status), None))
         return grads, status
 
     def gradients(self, cache, dy):
