@@ -343,9 +343,10 @@ struct sp_workspace {
   // row) the next predictor applies, or -1: settle_accept() writes it at once for anything
   // else that reads the state or the history rows.
   int pending_accept = -1;
-  // A single run's Adams attempt phase (table uploads, predict, source, correct, the norms'
-  // read-back), captured once and replayed: its launches and arguments are the same for
-  // every attempt, the tables' contents change in the pinned buffers the copies read
+  // A single run's Adams attempt phase (tables' fetch, predict, source, correct), captured once
+  // and replayed: its launches and arguments are the same for every attempt, the tables'
+  // contents change in the pinned buffer the fetch reads.  48 attempts of the gradient run:
+  // 5.05 ms; launched kernel by kernel, chained as in the graph, 5.30 ms.
   cudaGraph_t attempt_graph = nullptr;
   cudaGraphExec_t attempt_exec = nullptr;
   static constexpr int kStageSlots = 10;
@@ -1495,7 +1496,8 @@ static void check_column(const double* h_norms, double* d_norms, cudaStream_t s)
 
 // The attempt phase of a single run's Adams attempt, issued on the workspace's stream: the
 // step's two stage slots and tables from the pinned buffers, the predictor, the source at the
-// predicted field, the corrector with its reduction, the norms to the pinned host buffer.
+// predicted field, the corrector with its reduction, whose last block writes the norms to the
+// pinned host buffer.
 static void issue_attempt(sp_workspace* ws, const StepArgs& a) {
   // the trial's table and the step's two stage slots, contiguous on both sides
   static_assert((sizeof(AdamsDev) + 2 * sizeof(StageScalarsDev)) % 16 == 0, "fetched in 16-byte units");
@@ -1510,7 +1512,7 @@ static void issue_attempt(sp_workspace* ws, const StepArgs& a) {
 
 // One Adams attempt of a single run; returns accepted.  Without per-kernel timing the attempt
 // phase is a CUDA graph, captured on the first attempt and replayed (one launch instead of
-// nine); the copies out of the pinned tables are released by an event recorded after it.
+// six); the pinned tables are released by an event recorded after it.
 static bool adams_attempt(sp_session* S, double dz, double end, bool kink, bool fixed) {
   sp_workspace* ws = S->ws;
   Pending pd = prepare_attempt(S, dz, end, kink, fixed);
