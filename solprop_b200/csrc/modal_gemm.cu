@@ -537,11 +537,13 @@ __global__ void __launch_bounds__(256, 2) k_gemm_f64(const double* __restrict__ 
 // tiles divide them, each split at least 8 slabs long
 int f64_splits(int tiles, int slabs) { return std::max(1, std::min(4 * 148 / tiles, slabs / 8)); }
 int f64_tiles(int n_modes, int n_to) { return ((n_to + kFN - 1) / kFN) * ((n_modes + kFM - 1) / kFM); }
-// the tcgen05 projection's: CTAs for two waves, and no accumulator longer than 32 slices (2 048
-// nodes), whose error grows with the length of the sum (kTerms)
+// the tcgen05 projection's: CTAs for four waves of at least 4 slices, and no accumulator longer
+// than 32 slices (2 048 nodes): its error grows with the length of the sum (kTerms).  Two waves are
+// as fast, but their sums are twice as long: 1.0e-6 from 64 bits on a fibre where four leave
+// about 5e-7 (3 600 nodes, rows of 4 096: 5.0e-7).
 int split3_splits(int tiles, int k_slices) {
   int s = 1;
-  while ((tiles * s < 2 * 148 && k_slices / (2 * s) >= 4) || k_slices > 32 * s) s *= 2;
+  while ((tiles * s < 4 * 148 && k_slices / (2 * s) >= 4) || k_slices > 32 * s) s *= 2;
   return s;
 }
 int mode_tile(int n_modes) { return n_modes <= 32 ? 32 : 64; }
