@@ -316,7 +316,7 @@ struct sp_workspace {
     DevBuf<float> t_window, t_window_d, synthesis, projection, rate_coeff, taps, proj;
     DevBuf<float> node_field, node_streams;
     DevBuf<ChannelTableT<float>> channels;
-    DevBuf<float2> env_twiddles, raman_table, row_outer, row_inner;
+    DevBuf<float2> raman_table, row_outer, row_inner;
   } f32;
   DevBuf<unsigned char> active, norm;
   DevBuf<StageScalarsDev> stage;   // kStageSlots slots
@@ -718,7 +718,6 @@ static EnvModalArgsT<R> env_modal_args(const sp_workspace* ws, const double2* la
   ea.n_components = d.n_pol_transform;
   ea.raman_kernels = P.raman_kernels;
   if constexpr (sizeof(R) == 8) {
-    ea.twiddles_r = ws->env_twiddles.p;
     ea.raman_table = ws->raman_table.p;
     ea.outer_twiddles = ws->row_outer.p;
     ea.inner_twiddles = ws->row_inner.p;
@@ -727,7 +726,6 @@ static EnvModalArgsT<R> env_modal_args(const sp_workspace* ws, const double2* la
     ea.projected = ws->proj.p;
     ea.spectra = ws->spectra.p;
   } else {
-    ea.twiddles_r = ws->f32.env_twiddles.p;
     ea.raman_table = ws->f32.raman_table.p;
     ea.outer_twiddles = ws->f32.row_outer.p;
     ea.inner_twiddles = ws->f32.row_inner.p;
@@ -947,10 +945,14 @@ static void build_workspace(sp_workspace* ws) {
   // twiddles exp(-2 pi i m / n_to), m < n_to/2, in long double, rounded once
   std::vector<double2> tw(d.n_to / 2);
   const long double two_pi = 6.283185307179586476925286766559005768L;
-  for (int m = 0; m < d.n_to / 2; ++m) {
-    long double ang = two_pi * (long double)m / (long double)d.n_to;
-    tw[m] = make_double2((double)cosl(ang), (double)(-sinl(ang)));
-  }
+  auto root = [&](int m, int n) {
+    const long double ang = two_pi * (long double)m / (long double)n;
+    return make_double2((double)cosl(ang), (double)(-sinl(ang)));
+  };
+  // the doubled grid's table (envelope route, Raman), whose even entries are the grid's
+  std::vector<double2> tw2(d.grid_kind == 1 || d.raman_enabled ? d.n_to : 0);
+  for (int m = 0; m < (int)tw2.size(); ++m) tw2[m] = root(m, 2 * d.n_to);
+  for (int m = 0; m < d.n_to / 2; ++m) tw[m] = tw2.empty() ? root(m, d.n_to) : tw2[2 * m];
   ws->twiddles.upload(tw.data(), tw.size(), s);
   ws->omega.upload(P.omega.data(), d.n_omega, s);
   ws->omega_window.upload(P.omega_window.data(), d.n_omega, s);
@@ -1071,19 +1073,8 @@ static void build_workspace(sp_workspace* ws) {
     ws->launches = 4 + synthesis + 2 * streams + (d.raman_enabled ? 2 : 0);
   }
   if (ws->precision == SP_PRECISION_MIXED) build_mixed(ws, tw, rc, taps);
-  if (d.grid_kind == 1 || d.raman_enabled) {  // the doubled grid's table: envelope route, Raman
-    std::vector<double2> tw2(d.n_to);
-    for (int m = 0; m < d.n_to; ++m) {
-      long double ang = two_pi * (long double)m / (long double)(2 * d.n_to);
-      tw2[m] = make_double2((double)cosl(ang), (double)(-sinl(ang)));
-    }
+  if (!tw2.empty()) {
     ws->env_twiddles.upload(tw2.data(), tw2.size(), s);
-    if (ws->precision == SP_PRECISION_MIXED) {
-      std::vector<float2> tw2f(tw2.size());
-      for (size_t m = 0; m < tw2.size(); ++m) tw2f[m] = make_float2((float)tw2[m].x, (float)tw2[m].y);
-      ws->f32.env_twiddles.upload(tw2f.data(), tw2f.size(), s);
-      CUDA_CHECK(cudaStreamSynchronize(s));  // the host copy goes with this scope
-    }
     if (d.raman_enabled) ws->raman_undamped.upload(P.raman_undamped.data(), P.raman_undamped.size(), s);
     if (!P.raman_weights.empty()) ws->raman_weights.upload(P.raman_weights.data(), P.raman_weights.size(), s);
     if (d.raman_enabled && (d.grid_kind == 0 || ws->gemm))

@@ -264,7 +264,6 @@ struct EnvModalArgsT {
   const double2* lab;             // (n_cols, n_omega)
   const long long* crop;          // (n_omega): coarse bin -> fine bin
   const double2* twiddles;        // exp(-2 pi i m / (2 n_to)), m < n_to
-  const cplx<R>* twiddles_r;      // the same table in the form's type
   const double* t_window;         // (n_to)
   const double* alpha;            // the in-stage absorber's rate (n_to), or null
   double* modal_t;                // (n_cols, 2 n_to): a(t)

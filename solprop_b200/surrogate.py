@@ -132,29 +132,6 @@ def transpose_bf16(x, rows_pad: int):
     return out
 
 
-def convert_batch(xs, copies=None, transposes=None):
-    """BF16 copies (rows zero-padded to ``copies[q]`` columns) and transposes (zero-padded to
-    ``transposes[q]`` source rows) of FP32 or BF16 matrices, eight to a launch, either list
-    None; returns the two lists."""
-    import torch
-
-    n = len(xs)
-    if n > 8:
-        head = convert_batch(xs[:8], copies and copies[:8], transposes and transposes[:8])
-        tail = convert_batch(xs[8:], copies and copies[8:], transposes and transposes[8:])
-        return tuple(None if a is None else a + b for a, b in zip(head, tail))
-    new = lambda rows, cols, x: torch.empty((rows, cols), dtype=torch.bfloat16, device=x.device)  # noqa: E731
-    out = [new(x.shape[0], c, x) for x, c in zip(xs, copies)] if copies else None
-    out_t = [new(x.shape[1], r, x) for x, r in zip(xs, transposes)] if transposes else None
-    ints = lambda v: (C.c_int * n)(*v)  # noqa: E731
-    none = [None] * n
-    _check(_bind().sp_mlp_convert_batch(
-        n, int(xs[0].dtype == torch.bfloat16), _pointers(xs), ints(x.shape[0] for x in xs),
-        ints(x.shape[1] for x in xs), ints(x.stride(0) for x in xs), _pointers(out or none), ints(copies or [0] * n),
-        _pointers(out_t or none), ints(transposes or [0] * n), None))
-    return out, out_t
-
-
 def _pointers(tensors):
     return (C.c_void_p * len(tensors))(*[None if t is None else t.data_ptr() for t in tensors])
 

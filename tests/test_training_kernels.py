@@ -1,6 +1,8 @@
 """The surrogate's fused training kernels against plain PyTorch in 64 bits, at batches that fill
 no tile of rows and layers at both ends of the sizes they take."""
 
+import ctypes as C
+
 import pytest
 
 from solprop_b200 import _lib, surrogate
@@ -49,7 +51,15 @@ def test_batched_conversion_and_adam():
 
     g = torch.Generator(device="cuda").manual_seed(3)
     xs = [torch.randn(r, c, device="cuda", generator=g) for r, c in ((1, 6), (33, 64), (512, 6), (100, 512))]
-    copies, transposes = surrogate.convert_batch(xs, [64, 64, 64, 512], [64, 64, 512, 128])
+    wide, pads = [64, 64, 64, 512], [64, 64, 512, 128]
+    new = lambda r, c: torch.full((r, c), float("nan"), dtype=torch.bfloat16, device="cuda")  # noqa: E731
+    copies = [new(x.shape[0], c) for x, c in zip(xs, wide)]
+    transposes = [new(x.shape[1], r) for x, r in zip(xs, pads)]
+    ints = lambda v: (C.c_int * 4)(*v)  # noqa: E731
+    pointers = lambda ts: (C.c_void_p * 4)(*[t.data_ptr() for t in ts])  # noqa: E731
+    _lib.check(_lib.library().sp_mlp_convert_batch(
+        4, 0, pointers(xs), ints(x.shape[0] for x in xs), ints(x.shape[1] for x in xs), ints(x.stride(0) for x in xs),
+        pointers(copies), ints(wide), pointers(transposes), ints(pads), None))
     for x, c, t in zip(xs, copies, transposes):
         r, k = x.shape
         assert torch.equal(c[:, :k], x.bfloat16()) and not c[:, k:].any()
