@@ -60,62 +60,10 @@ struct GemmBatch {
   int count;
 };
 
-// ---- the GELU x Phi(x) of two values, in packed FP32 instructions: the epilogue's issue slots
-// are what a hidden layer's tile costs.  With z = |x| / sqrt 2 it is max(x, 0) - |x| erfc(z) / 2,
-// and erfc(z) / 2 = exp(-z^2) t q(t) with t = 1 / (1 + 0.37 z) and q of degree 8, fitted to
-// exp(z^2) erfc(z) (least squares weighted towards the largest relative error, 6e-9).  Against
-// x Phi(x) in 64 bits over [-8, 8]: 2.4e-7 at most, 4.4e-8 rms, and for x < -1 within 3e-6 of the
-// value itself; 0.5 x (1 + erff(x / sqrt 2)): 4.5e-7, 5.7e-8, and no correct digit left at x = -6.
-using Pair = unsigned long long;
-__device__ __forceinline__ Pair pack(float a, float b) {
-  Pair r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpack(Pair p, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p));
-}
-__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
-  Pair r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
-  Pair r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ Pair both(float a) { return pack(a, a); }
-__device__ __forceinline__ float fast_reciprocal(float a) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
-  return r;
-}
-__device__ __forceinline__ float fast_exp2(float a) {
-  float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
-  return r;
-}
-__device__ __forceinline__ void gelu2(float& x0, float& x1) {
-  const Pair x = pack(x0, x1), a = pack(fabsf(x0), fabsf(x1));
-  float d0, d1;
-  unpack(fma2(a, both(0.26162951f), both(1.0f)), d0, d1);  // 0.37 / sqrt 2
-  const Pair t = pack(fast_reciprocal(d0), fast_reciprocal(d1));
-  Pair p = both(0.032264236f);
-  p = fma2(p, t, both(-0.15801775f));
-  p = fma2(p, t, both(0.25675202f));
-  p = fma2(p, t, both(-0.15814187f));
-  p = fma2(p, t, both(0.16632225f));
-  p = fma2(p, t, both(0.048480004f));
-  p = fma2(p, t, both(0.10439319f));
-  p = fma2(p, t, both(0.10352958f));
-  p = fma2(p, t, both(0.10441834f));
-  float e0, e1, h0, h1;
-  unpack(mul2(mul2(x, x), both(-0.72134752f)), e0, e1);  // -log2(e) / 2
-  unpack(mul2(mul2(a, pack(fast_exp2(e0), fast_exp2(e1))), mul2(p, t)), h0, h1);
-  x0 = fmaxf(x0, 0.0f) - h0;
-  x1 = fmaxf(x1, 0.0f) - h1;
-}
+// The GELU is the other products' (k_mlp_gemm), in the same FP32 operations.  A rational fit in packed
+// FP32 instructions was a tenth faster (16 384 points of five members: 518 us against 569) but twice
+// as far from x Phi(x) for small arguments, and gave NaN for +infinity.
+__device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -289,7 +237,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         if (epilogue == 2) {
 #pragma unroll
-          for (int j = 0; j < 32; j += 2) gelu2(v[j], v[j + 1]);
+          for (int j = 0; j < 32; ++j) v[j] = gelu(v[j]);
         }
         if (C) {
           // FP32 rows: lane `lane` (row) writes its eight 16-byte units, unit s of row rr at
@@ -310,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (C16) {
           if (epilogue == 3) {  // training: the pre-activation above, its GELU here
 #pragma unroll
-            for (int j = 0; j < 32; j += 2) gelu2(v[j], v[j + 1]);
+            for (int j = 0; j < 32; ++j) v[j] = gelu(v[j]);
           }
           // BF16 rows of 64 bytes: unit s (eight values) of row rr at slot s ^ ((rr >> 1) & 3)
           // of that row's four; lanes 4 i .. 4 i + 3 then take row 8 k + i's units

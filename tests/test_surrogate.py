@@ -94,6 +94,40 @@ def test_tcgen05_gemm_matches_bf16_oracle(shape):
 
 
 @gpu
+def test_tcgen05_gelu_epilogue_against_64_bits():
+    """The hidden layers' GELU alone (products of zeros, the argument in the bias) against
+    x Phi(x) in 64 bits.  The bound, 0.5 x (1 + erff(x c)) in FP32: two units in the last place
+    of erff (2^-22 of its value), the argument's two roundings (2^-23 z erf'(z)), the sum's
+    (2^-24 where it is below 2) and the two products' (2^-23 of the result)."""
+    from solprop_b200 import surrogate as S
+
+    torch = _torch()
+    grid = np.linspace(-8, 8, 8192 - 1024).astype(np.float32)
+    far = np.geomspace(1e-30, 1e3, 512).astype(np.float32)
+    x = np.concatenate([grid, far, -far])
+    x[-1], x[-2], x[-3] = np.inf, np.float32(1e30), np.nan
+    a16 = torch.zeros((5, 64), dtype=torch.bfloat16, device="cuda")
+    w16 = torch.zeros((x.size, 64), dtype=torch.bfloat16, device="cuda")
+    out, pre = torch.empty((5, x.size), device="cuda"), torch.empty((5, x.size), device="cuda")
+    half, trained = (torch.empty((5, x.size), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    bias = torch.tensor(x, device="cuda")
+    S.gemm_tc(a16, w16, out=out, out16=half, bias=bias, epilogue=2)
+    status = S.gemm_tc(a16, w16, out=pre, out16=trained, bias=bias, epilogue=3)
+    assert int(status.item()) == 0
+    got, z = out.double().cpu(), torch.tensor(x.astype(np.float64) / np.sqrt(2.0))
+    assert torch.equal(got[:, -1], torch.full((5,), np.inf, dtype=torch.float64)) and torch.isnan(got[:, -3]).all()
+    finite = torch.isfinite(z)
+    got, z = got[:, finite], z[finite]
+    erf, slope = torch.erf(z), 2 / np.sqrt(np.pi) * torch.exp(-z * z) * z.abs()
+    want = z / np.sqrt(2.0) * torch.erfc(-z)
+    bound = z.abs() / np.sqrt(2.0) * (2**-22 * erf.abs() + 2**-23 * slope + 2**-24) + 2**-23 * want.abs()
+    assert bool(((got - want).abs() <= bound + 1e-45).all())
+    assert torch.equal(pre[:, :-3], bias[:-3].expand(5, -1))
+    for h in (half, trained):
+        assert torch.equal(h[:, finite], out.bfloat16()[:, finite])
+
+
+@gpu
 def test_inference_on_tcgen05_matches_the_training_path():
     from solprop_b200 import surrogate as S
 
