@@ -140,6 +140,22 @@ def _pad64(n: int) -> int:
     return -(-n // 64) * 64
 
 
+def _rows(t, cols: int, dense: bool = False):
+    """A 2-D tensor as the native passes read it, `cols` values a row (`dense`: no gap between
+    rows), and its row pitch: itself, or a copy (short rows zero-padded, long ones cut) where it
+    is laid out otherwise.  The copy is made on the stream the passes run on."""
+    import torch
+
+    unit = t.shape[1] == cols and (cols == 1 or t.stride(1) == 1)
+    if not unit or (t.shape[0] > 1 and (t.stride(0) < cols or (dense and t.stride(0) != cols))):
+        with torch.cuda.stream(torch.cuda.default_stream(t.device)):
+            copy = torch.zeros((t.shape[0], cols), dtype=t.dtype, device=t.device)
+            width = min(cols, t.shape[1])
+            copy[:, :width] = t[:, :width]
+        t = copy
+    return t, t.stride(0) if t.shape[0] > 1 else cols
+
+
 # ------------------------------------------------------------------ features and targets
 def features(points) -> np.ndarray:
     """The six inputs of each point, each mapped onto [-1, 1] over the scan's ranges."""
@@ -246,9 +262,15 @@ class Perceptron:
     def forward_tc(self, x, keep: bool = False, status=None):
         """The training's forward pass on the tcgen05 products (``gemm_tc``): BF16 operands,
         FP32 accumulation; the hidden layers write their pre-activations in FP32 and their
-        activations in BF16 (epilogue 3).  Returns the output, the cache and the status."""
+        activations in BF16 (epilogue 3).  The first product takes K padded to 64, so inputs of
+        any width that pads to the same are taken: missing columns are zeros, columns beyond the
+        weights' meet none.  Returns the output, the cache and the status."""
         import torch
 
+        k0 = self.weights[0].shape[1]
+        if _pad64(x.shape[1]) != _pad64(k0):
+            raise ValueError(f"forward_tc: {x.shape[1]} inputs for weights of {k0}")
+        rows, ldx = _rows(x, k0)
         m, hidden = x.shape[0], self.weights[:-1]
         pre = [torch.empty((m, w.shape[0]), dtype=torch.float32, device=self.device) for w in hidden]
         act = [torch.empty((m, w.shape[0]), dtype=torch.bfloat16, device=self.device) for w in hidden]
@@ -257,7 +279,7 @@ class Perceptron:
             status = torch.zeros(1, dtype=torch.int32, device=x.device)
         sizes, scratch = self._training_pass(m)
         _check(_bind().sp_mlp_training_forward(
-            *sizes, _pointers(self.weights), _pointers(self.biases), _ptr(x), x.stride(0), _pointers(pre),
+            *sizes, _pointers(self.weights), _pointers(self.biases), _ptr(rows), ldx, _pointers(pre),
             _pointers(act), _ptr(out), _ptr(scratch), scratch.numel(), _ptr(status), None))
         kept = pre if keep else [None] * len(pre)
         return out, list(zip([x, *act], [*kept, None])), status
@@ -278,18 +300,34 @@ class Perceptron:
         below the products' 256-column tiles, in a kernel of its own.  Each layer's dz, its
         copies and its bias gradient come from one pass, the transposes of the weights and of
         the activations from one launch each, and the weight gradients of one shape share a
-        launch.  Returns (grads, status)."""
+        launch.  The cache is forward_tc's, or forward's (FP32 activations, rounded here).
+        Returns (grads, status)."""
         import torch
 
+        m = dy.shape[0]
+        if tuple(dy.shape) != (m, self.weights[-1].shape[0]):
+            raise ValueError(f"gradients_tc: dy {tuple(dy.shape)} for {self.weights[-1].shape[0]} outputs")
+        acts, pres = [], []
+        for i, w in enumerate(self.weights):
+            a, pre = cache[i]
+            if tuple(a.shape) != (m, w.shape[1]) or (pre is not None and pre.numel() != m * w.shape[0]):
+                raise ValueError(f"gradients_tc: layer {i}, weights {tuple(w.shape)}, a batch of {m}: inputs "
+                                 f"{tuple(a.shape)}, pre-activations {None if pre is None else tuple(pre.shape)}")
+            a, lda = _rows(a, w.shape[1], dense=i > 0)
+            if i == 0:
+                x, ldx = a, lda
+            else:
+                acts.append(a if a.dtype == torch.bfloat16 else to_bf16(a, w.shape[1]))
+            pres.append(pre)
+        dy, _ = _rows(dy, dy.shape[1], dense=True)
         grads = [torch.empty_like(p) for p in self.params]
         if status is None:
             status = torch.zeros(1, dtype=torch.int32, device=dy.device)
-        x = cache[0][0]
-        sizes, scratch = self._training_pass(dy.shape[0])
+        sizes, scratch = self._training_pass(m)
         _check(_bind().sp_mlp_training_backward(
-            *sizes, _pointers(self.weights), _ptr(x), x.stride(0), _pointers([pre for _, pre in cache]),
-            _pointers([a for a, _ in cache[1:]]), _ptr(dy), _pointers(grads[::2]), _pointers(grads[1::2]),
-            _ptr(scratch), scratch.numel(), _ptr(status), None))
+            *sizes, _pointers(self.weights), _ptr(x), ldx, _pointers(pres), _pointers(acts),
+            _ptr(dy), _pointers(grads[::2]), _pointers(grads[1::2]), _ptr(scratch), scratch.numel(), _ptr(status),
+            None))
         return grads, status
 
     def gradients(self, cache, dy):
@@ -320,6 +358,7 @@ class Perceptron:
     def adam(self, grads, lr: float, betas=(0.9, 0.999), eps: float = 1e-8):
         lib = _bind()
         self.step += 1
+        grads = list(grads)[:len(self.params)]
         for s in range(0, len(grads), 16):
             part = slice(s, s + 16)
             sizes = (C.c_size_t * len(grads[part]))(*[p.numel() for p in self.params[part]])

@@ -72,3 +72,128 @@ def test_batched_conversion_and_adam():
                                               1e-3, 0.9, 0.999, 1e-8, 1, None))
     for a, b in zip(net.params + net.m1 + net.m2, one.params + one.m1 + one.m2):
         assert torch.equal(a, b)
+
+
+# ---- what the native passes are handed: they read rows by the weights' sizes alone, so a tensor
+# of another shape is refused before the call (no GPU: a library that only records its calls)
+class _Recorder:
+    def __init__(self):
+        self.calls = {}
+
+    def __getattr__(self, name):
+        def call(*args):
+            self.calls[name] = args
+            return 256 if name.endswith("scratch") else 0
+        return call
+
+
+def _cpu_member(sizes=(6, 32, 32, 16)):
+    import torch
+
+    net = object.__new__(surrogate.Perceptron)
+    net.device, net.step = torch.device("cpu"), 0
+    net.weights = [torch.zeros(b, a) for a, b in zip(sizes[:-1], sizes[1:])]
+    net.biases = [torch.zeros(b) for b in sizes[1:]]
+    net.params = [t for pair in zip(net.weights, net.biases) for t in pair]
+    net.m1, net.m2 = ([torch.zeros_like(t) for t in net.params] for _ in range(2))
+    return net
+
+
+@pytest.fixture
+def recorder(monkeypatch):
+    lib = _Recorder()
+    monkeypatch.setattr(surrogate, "_bind", lambda: lib)
+    return lib
+
+
+def _cache(net, m):
+    import torch
+
+    dims = [w.shape for w in net.weights]
+    return [(torch.zeros(m, k, dtype=torch.bfloat16 if i else torch.float32),
+             torch.zeros(m, n) if i + 1 < len(dims) else None) for i, (n, k) in enumerate(dims)]
+
+
+@pytest.mark.parametrize("wrong", ["dy narrow", "dy wide", "dy short", "dy long", "inputs", "activations", "rows",
+                                   "pre-activations", "cache"])
+def test_backward_refuses_other_shapes(recorder, wrong):
+    import torch
+
+    net, m = _cpu_member(), 40
+    cache, dy = _cache(net, m), torch.zeros(m, 16)
+    net.gradients_tc(cache, dy)
+    assert "sp_mlp_training_backward" in recorder.calls
+    recorder.calls.clear()
+    if wrong.startswith("dy"):
+        dy = {"dy narrow": torch.zeros(m, 15), "dy wide": torch.zeros(m, 17), "dy short": torch.zeros(m - 1, 16),
+              "dy long": torch.zeros(m + 1, 16)}[wrong]
+    elif wrong == "inputs":
+        cache[0] = (torch.zeros(m, 5), cache[0][1])
+    elif wrong == "activations":
+        cache[2] = (cache[2][0][:, :31], cache[2][1])
+    elif wrong == "rows":
+        cache[1] = (cache[1][0][:-1], cache[1][1])
+    elif wrong == "pre-activations":
+        cache[1] = (cache[1][0], cache[1][1][:-1])
+    else:
+        del cache[2]
+    with pytest.raises((ValueError, IndexError)):
+        net.gradients_tc(cache, dy)
+    assert "sp_mlp_training_backward" not in recorder.calls
+
+
+def test_forward_refuses_inputs_of_another_padded_width(recorder):
+    import torch
+
+    net = _cpu_member()
+    net.forward_tc(torch.zeros(9, 6))
+    assert "sp_mlp_training_forward" in recorder.calls
+    recorder.calls.clear()
+    for width in (0, 65):
+        with pytest.raises(ValueError):
+            net.forward_tc(torch.zeros(9, width))
+    assert "sp_mlp_training_forward" not in recorder.calls
+
+
+def test_adam_takes_no_more_gradients_than_parameters(recorder):
+    import torch
+
+    net = _cpu_member()
+    grads = [torch.zeros_like(p) for p in net.params]
+    net.adam(iter(grads + [torch.zeros(3)]), 1e-3)
+    count, pointers = recorder.calls["sp_mlp_adam_batch"][:2]
+    assert count == len(net.params) == len(pointers)
+
+
+@pytest.mark.gpu
+def test_training_pass_over_other_layouts():
+    """Inputs of fewer or more columns, views and repeated rows, and the FP32 path's cache, against
+    the same values laid out plainly: the same bits."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    net = surrogate.Perceptron(3)
+    six = torch.randn(40, 6, device="cuda", generator=g)
+    five = six.clone()
+    five[:, 5] = 0
+    seven = torch.cat([six, torch.ones(40, 1, device="cuda")], 1)
+    repeated = six[:1].expand(40, 6)
+    plain = {name: net.forward_tc(x.contiguous(), keep=True) for name, x in
+             (("six", six), ("five", five), ("repeated", repeated))}
+    for name, x in (("five", five[:, :5].contiguous()), ("five", six[:, :5]), ("six", seven), ("six", seven[:, :6]),
+                    ("six", six.T.contiguous().T), ("repeated", repeated)):
+        out, _, status = net.forward_tc(x, keep=True)
+        assert int(status.item()) == 0 and torch.equal(out, plain[name][0]), (name, x.shape, x.stride())
+    dy = torch.randn(40, surrogate.N_OUT, device="cuda", generator=g)
+    _, cache, _ = plain["six"]
+    want, _ = net.gradients_tc(cache, dy)
+    wide = torch.zeros(40, surrogate.N_OUT + 4, device="cuda")
+    wide[:, :surrogate.N_OUT] = dy
+    strided = [(seven[:, :6], cache[0][1]), *cache[1:]]
+    for c, d in ((cache, wide[:, :surrogate.N_OUT]), (strided, dy)):
+        got, status = net.gradients_tc(c, d)
+        assert int(status.item()) == 0 and all(torch.equal(a, b) for a, b in zip(got, want))
+    _, fp32 = net.forward(six, keep=True)
+    want, _ = net.gradients_tc([(a if i == 0 else a.bfloat16(), pre) for i, (a, pre) in enumerate(fp32)], dy)
+    got, _ = net.gradients_tc(fp32, dy)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
