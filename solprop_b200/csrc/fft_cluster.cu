@@ -191,7 +191,7 @@ __device__ __forceinline__ void forward_cluster_body(const ForwardArgsT<R>& a, i
         Cx x[kBatch];
 #pragma unroll
         for (int g = 0; g < kBatch; ++g)
-          if (g0 + g < a.n_groups) x[g] = __ldg(rows + (size_t)(g0 + g) * group_stride + m);
+          if (g0 + g < a.n_groups) x[g] = __ldcg(rows + (size_t)(g0 + g) * group_stride + m);
 #pragma unroll
         for (int g = 0; g < kBatch; ++g) {
           if (g0 + g >= a.n_groups) break;

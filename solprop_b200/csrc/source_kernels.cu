@@ -132,7 +132,7 @@ __device__ __forceinline__ void forward_field_body(const ForwardArgsT<R>& a, int
         V x[kBatch];
 #pragma unroll
         for (int g = 0; g < kBatch; ++g)
-          if (g0 + g < a.n_groups) x[g] = __ldg(rows16 + (size_t)(g0 + g) * group_stride + v);
+          if (g0 + g < a.n_groups) x[g] = __ldcg(rows16 + (size_t)(g0 + g) * group_stride + v);
 #pragma unroll
         for (int g = 0; g < kBatch; ++g) {
           if (g0 + g >= a.n_groups) break;

@@ -68,6 +68,9 @@ __host__ __device__ __forceinline__ double2 to_d2(float2 v) { return make_double
 // for that one's end; and it lets the next be launched at once.  Every kernel of the chain
 // waits, so each sees the writes of all before it.  A kernel launched in the ordinary way
 // passes straight through.  It saves a launch's latency per kernel, about 1 us of 5.
+// Such a kernel runs beside the one that writes its inputs, and non-coherent loads are not ordered
+// after the wait: __ldg and const __restrict__ are for tables written at workspace creation alone,
+// what an earlier kernel of the chain wrote is read by plain loads or __ldcg.
 __device__ __forceinline__ void await_previous_kernel() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
