@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint64_t* drain = acc_empty + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
   __shared__ volatile int failed;
-  __shared__ int consumed;  // ring slices the products have taken (for the drain on failure)
+  __shared__ volatile int consumed;  // ring slices the products have taken (for the drain on failure)
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int n_k = K / kTK;
   const int tiles_n = N / kTN, per_product = tiles_n * ((M + kTM - 1) / kTM);
@@ -124,9 +124,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
 
+  long loads = 0;  // K slices asked for (thread 0)
   if (threadIdx.x == 0) {
     // producer: the K slices of every tile of this CTA, through the ring
-    long g = 0;
+    long& g = loads;
     for (int t = blockIdx.x; t < tiles && !failed; t += gridDim.x) {
       const int q = t / per_product, u = t % per_product;
       const int m0 = (u / tiles_n) * kTM, n0 = (u % tiles_n) * kTN;
@@ -144,9 +145,6 @@ __global__ void __launch_bounds__(kThreads, 1)
         tma_load_2d(stage + kABytes, &p.w[q], &full[s], k * kTK, n0);
       }
     }
-    // on failure: the loads still in flight land before the CTA leaves
-    if (failed)
-      for (long h = consumed; h < g; ++h) mbar_wait(&full[h % kStages], (uint32_t)(h / kStages) & 1);
   } else if (threadIdx.x == 32) {
     // the MMA issuer: tile i into accumulator i % 2 once the epilogue has read it
     long g = 0;
@@ -201,12 +199,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int j4 = 0; j4 < 8; ++j4) b4[j4] = __ldg(reinterpret_cast<const float4*>(bias + n0 + c) + j4);
       };
       if (bias) load_bias(slice * kEpilogueColumns);
-      const bool ok = mbar_wait(&acc_full[b], (it >> 1) & 1);
-      if (!ok || failed) {
+      if (!warp_agrees(mbar_wait(&acc_full[b], (it >> 1) & 1) && !failed)) {
         failed = 1;
         break;
       }
-      __syncwarp();
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = tmem + (uint32_t)b * kAccColumns + ((uint32_t)(quarter * 32) << 16);
       const int m_first = m0 + quarter * 32;
@@ -288,7 +284,12 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncwarp();  // warps 0 and 1 wait for their producing / issuing lane before the barrier
   __syncthreads();
   // the products issued (all of them, or those before a failure) are complete
-  if (threadIdx.x == 0 && !mbar_wait(drain, 0)) failed = 1;
+  if (threadIdx.x == 0) {
+    if (!mbar_wait(drain, 0)) failed = 1;
+    // on failure: the loads still in flight land before the CTA leaves
+    if (failed)
+      for (long h = consumed; h < loads; ++h) mbar_wait(&full[h % kStages], (uint32_t)(h / kStages) & 1);
+  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0)

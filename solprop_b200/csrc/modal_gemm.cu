@@ -115,8 +115,9 @@ __global__ void __launch_bounds__(kSynThreads, 1)
   fence_after();
   const uint32_t tmem = *tmem_slot;
 
+  int loads = 0;  // K slices asked for (thread 0)
   if (threadIdx.x == 0) {
-    int g = 0;
+    int& g = loads;
     for (int tile = first; tile < last && !failed; ++tile) {
       const int t0 = (tile / row_tiles) * kGM, r0 = (tile % row_tiles) * 128;
       for (int k = 0; k < n_k; ++k, ++g) {
@@ -133,8 +134,6 @@ __global__ void __launch_bounds__(kSynThreads, 1)
         }
       }
     }
-    if (failed)  // the loads in flight land before the CTA leaves
-      for (int h = consumed; h < g; ++h) mbar_wait(&full[h % kSynStages], (uint32_t)(h / kSynStages) & 1);
   } else if (threadIdx.x == 32) {
     constexpr uint32_t kIdescN = idesc_bf16(kGM, 128);
     int g = 0, it = 0;
@@ -174,11 +173,10 @@ __global__ void __launch_bounds__(kSynThreads, 1)
     int it = 0;
     for (int tile = first; tile < last; ++tile, ++it) {
       const int b = it % kSynAcc;
-      if (!mbar_wait(&acc_full[b], (uint32_t)(it / kSynAcc) & 1) || failed) {
+      if (!warp_agrees(mbar_wait(&acc_full[b], (uint32_t)(it / kSynAcc) & 1) && !failed)) {
         failed = 1;
         break;
       }
-      __syncwarp();
       fence_after();
       const int t = (tile / row_tiles) * kGM + quarter * 32 + lane, r0 = (tile % row_tiles) * 128 + half * 64;
       float* out = E + (size_t)r0 * n_t + t;
@@ -207,7 +205,11 @@ __global__ void __launch_bounds__(kSynThreads, 1)
   }
   __syncwarp();
   __syncthreads();
-  if (threadIdx.x == 0 && !mbar_wait(drain, 0)) failed = 1;
+  if (threadIdx.x == 0) {
+    if (!mbar_wait(drain, 0)) failed = 1;
+    if (failed)  // the loads in flight land before the CTA leaves
+      for (int h = consumed; h < loads; ++h) mbar_wait(&full[h % kSynStages], (uint32_t)(h / kSynStages) & 1);
+  }
   fence_before();
   __syncthreads();
   if (warp == 0) tmem_free_all(tmem);
@@ -298,8 +300,9 @@ __global__ void __launch_bounds__(kProThreads, 1)
   fence_after();
   const uint32_t tmem = *tmem_slot;  // the accumulators' BN columns (hi hi, the rest), then the stages'
 
+  int loads = 0;  // slices of W asked for (thread 0)
   if (threadIdx.x == 0) {
-    int g = 0;
+    int& g = loads;
     for (; g < total && !failed; ++g) {
       const int s = g % kProStages;
       if (g >= kProStages && !mbar_wait(&empty[s], (uint32_t)(g / kProStages - 1) & 1)) {
@@ -310,8 +313,6 @@ __global__ void __launch_bounds__(kProThreads, 1)
       mbar_expect_tx(&w_full[s], kStage);
       for (int p = 0; p < 3; ++p) tma_load_2d(stage + p * (BN * kGK * 2), &maps.b[p], &w_full[s], (ks0 + g) * kGK, m0);
     }
-    if (failed)  // the loads in flight land before the CTA leaves
-      for (int h = consumed; h < g; ++h) mbar_wait(&w_full[h % kProStages], (uint32_t)(h / kProStages) & 1);
   } else if (threadIdx.x == 32) {
     constexpr uint32_t kIdescN = idesc_bf16(kGM, BN);
     for (int g = 0; g < total && !failed; ++g) {
@@ -348,9 +349,10 @@ __global__ void __launch_bounds__(kProThreads, 1)
       float v[kGK];
 #pragma unroll
       for (int i = 0; i < kGK; ++i) v[i] = k0 + i < n_nodes ? __ldcs(column + (size_t)(k0 + i) * n_t) : 0.0f;
-      if (g >= kProStages && !mbar_wait(&empty[s], (uint32_t)(g / kProStages - 1) & 1)) failed = 1;
-      if (failed) break;
-      __syncwarp();
+      if (!warp_agrees((g < kProStages || mbar_wait(&empty[s], (uint32_t)(g / kProStages - 1) & 1)) && !failed)) {
+        failed = 1;
+        break;
+      }
       fence_after();
       const uint32_t a = tmem + ((uint32_t)(quarter * 32) << 16) + 2 * BN + (uint32_t)s * kProACols;
       uint32_t packed[kGK / 2];
@@ -368,6 +370,8 @@ __global__ void __launch_bounds__(kProThreads, 1)
   __syncwarp();
   __syncthreads();
   const bool ok = mbar_wait(done, 0);
+  if (threadIdx.x == 0 && (!ok || failed))  // the loads in flight land before the CTA leaves
+    for (int h = consumed; h < loads; ++h) mbar_wait(&w_full[h % kProStages], (uint32_t)(h / kProStages) & 1);
   __syncwarp();
   fence_after();
   if (warp >= 4 && warp < 8) {

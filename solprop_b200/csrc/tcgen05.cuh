@@ -51,6 +51,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   return false;
 }
 
+// One answer for a whole warp: each lane's wait ends by itself and each reads the CTA's failure flag
+// for itself, but what follows (tensor-memory loads and stores, .sync.aligned) takes the warp as
+// one, so the lanes go on or leave together.
+__device__ __forceinline__ bool warp_agrees(bool ok) { return __all_sync(0xffffffffu, ok); }
+
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
