@@ -199,13 +199,16 @@ __device__ __forceinline__ void node_output(const EnvModalArgsT<R>& a, int nc, d
                                             cplx<R>& py) {
   using C = cplx<R>;
   const R self = R(a.kerr_self), conj = R(a.kerr_conjugate);
+  const double2 dx = to_d2(x), dy = to_d2(y);
+  // without Kerr the cubic is of zeros (a field above 7e12 overflows it in FP32): selections, which
+  // the unrolled samples carry better than a branch
+  if (!a.kerr) x.x = x.y = y.x = y.y = R(0);
   R mod = x.x * x.x + x.y * x.y;
   C sq = cmul(x, x);
   if (nc == 2) {
     mod += y.x * y.x + y.y * y.y;
     sq = cadd(sq, cmul(y, y));
   }
-  const double2 dx = to_d2(x), dy = to_d2(y);
   const double2 kx = to_d2(cadd(cscale(self * mod, x), cscale(conj, cmul(sq, cconj(x)))));
   const double rx = u + v;
   px = to_c<C>(make_double2(gate * fma(factor, kx.x, fma(rx, dx.x, w * dy.x)),

@@ -44,6 +44,19 @@ def test_source_matches_oracle(n_to, form, precision, bound):
     assert rel(ws.source(lab, 0.0), S.lab_source(rec, lab, 0.0)) < bound
 
 
+# Raman alone on a field whose cube overflows FP32 (above 7e12): no cubic is formed
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["tensor", "trace", "scalar"])
+@pytest.mark.parametrize("n_to", [512, 16384])
+def test_strong_field_without_kerr(n_to, form):
+    rec = dataclasses.replace(_record(n_to, form), kerr_enabled=False)
+    lab = rec.launch_field()
+    peak = np.abs(rec.synthesis @ np.fft.ifft(lab.reshape(rec.n_modes, -1), axis=-1)).max()
+    lab = lab * (2e13 / peak)
+    ws = _lib.Workspace(_lib.Problem(rec), 0, "mixed")
+    assert rel(ws.source(lab, 0.0), S.lab_source(rec, lab, 0.0)) < 2e-6
+
+
 # the products: mode counts about the projections' 32- and 64-wide tiles and the synthesis's 16-
 # and 64-wide K slices, rows of nodes that fill neither a tile nor a K slice
 @pytest.mark.gpu
