@@ -57,6 +57,36 @@ def test_strong_field_without_kerr(n_to, form):
     assert rel(ws.source(lab, 0.0), S.lab_source(rec, lab, 0.0)) < 2e-6
 
 
+# Two drives share a complex row: neighbouring nodes' traces, and one node's difference and
+# coherence.  A mode of its own on each, fields 1e4 apart (drives 1e8), a continuous wave beside a
+# pulse, or nothing at all beside one: the error of every mode's source against its own norm
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision, bound", [("fp64", 1e-13), ("mixed", 2e-6)])
+@pytest.mark.parametrize("form, rows", [("scalar", (2, 3)), ("trace", (4, 6)), ("tensor", (4, 6)), ("tensor", (4, 5))])
+@pytest.mark.parametrize("first", ["pulse", "continuous", "none"])
+@pytest.mark.parametrize("n_to", [512, 4096, 8192, 16384])
+def test_uneven_drives_of_one_row(n_to, first, form, rows, precision, bound):
+    rec = _record(n_to, form)
+    synthesis, projection = np.zeros((rec.synthesis.shape[0], 2)), np.zeros((2, rec.synthesis.shape[0]))
+    for mode, row in enumerate(rows):
+        synthesis[row, mode], projection[mode, row] = abs(rec.synthesis).max(), abs(rec.projection).max()
+    rec = dataclasses.replace(
+        rec, n_modes=2, phi_terms=rec.phi_terms[:, :2], prefactor_terms=rec.prefactor_terms[:, :2], synthesis=synthesis,
+        projection=projection, projection_coarse=projection, kerr_enabled=False, absorber_scheme="none",
+        temporal_absorber_fine=None, field0=rec.field0[:2])
+    lab = rec.launch_field()
+    lab[1] = 1e-4 * lab[0]
+    if first == "continuous":
+        peak = abs(lab[0]).argmax()
+        lab[0], lab[0].flat[peak] = 0.0, abs(lab[0]).sum()
+    elif first == "none":
+        lab[0] = 0.0
+    ws = _lib.Workspace(_lib.Problem(rec), 0, precision)
+    got, want = ws.source(lab, 0.0), S.lab_source(rec, lab, 0.0)
+    for mode in range(2):
+        assert np.linalg.norm(got[mode] - want[mode]) <= bound * np.linalg.norm(want[mode]), mode
+
+
 # the products: mode counts about the projections' 32- and 64-wide tiles and the synthesis's 16-
 # and 64-wide K slices, rows of nodes that fill neither a tile nor a K slice
 @pytest.mark.gpu
