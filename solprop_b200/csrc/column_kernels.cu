@@ -262,7 +262,7 @@ __device__ __forceinline__ double window_prefix(const R (&inc)[kPer], double (&P
 // exactly n_blocks tickets, so ticket / n_blocks numbers the evaluation (its epoch) and the
 // ready flags need no reset: a tile's flag reads 2 e + 1 once its exposure sums of
 // evaluation e are published and 2 e + 2 once its current sums are.
-constexpr long kSpinLimit = 1L << 20;  // polls of one flag before the wait gives up
+constexpr long kSpinLimit = 1L << 21;  // polls of one flag, 32 ns apart, before the wait gives up
 
 __device__ __forceinline__ int load_acquire(const int* p) {
   int v;

@@ -34,3 +34,10 @@ def test_whole_warp_roles_leave_as_one(name, count):
         assert not re.search(r"for \([^\n]*failed[^\n]*\)", role)
         # once every role has ended, the loads asked for and not taken land before the CTA leaves
         assert re.search(r"for \(\w+ h = consumed; h < loads; \+\+h\) mbar_wait", ending)
+
+
+def test_column_hand_over_waits_long_enough():
+    """A tile gives an earlier one at least 2^26 ns: polls times the sleep between them."""
+    text = (CSRC / "column_kernels.cu").read_text()
+    limit = int(re.search(r"kSpinLimit = 1L << (\d+);", text).group(1))
+    assert (1 << limit) * int(re.search(r"__nanosleep\((\d+)\)", text).group(1)) >= 1 << 26
