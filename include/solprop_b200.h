@@ -458,7 +458,7 @@ sp_status sp_mlp_first_layer_backward(const float* dA, const float* pre, const f
  * k[i]) with k[i + 1] = n[i], on the tcgen05 products (their rules on n and k; k[0] is free): forward
  * writes pre[i] (FP32) and act[i] (BF16) of the hidden layers and out; backward reads them (pre[i]
  * NULL: no GELU) and writes every dW and db.  scratch: sp_mlp_training_scratch bytes of device memory. */
-#define SP_MLP_MAX_LAYERS 16
+#define SP_MLP_MAX_LAYERS 64
 size_t sp_mlp_training_scratch(int layers, int M, const int* n, const int* k);
 sp_status sp_mlp_training_forward(int layers, int M, const int* n, const int* k, const float* const* W,
                                   const float* const* bias, const float* x, int ldx, float* const* pre,

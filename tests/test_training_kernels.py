@@ -197,3 +197,83 @@ def test_training_pass_over_other_layouts():
     want, _ = net.gradients_tc([(a if i == 0 else a.bfloat16(), pre) for i, (a, pre) in enumerate(fp32)], dy)
     got, _ = net.gradients_tc(fp32, dy)
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+# ---- the native passes themselves, beyond the surrogate's own network: one layer, a first layer
+# wider than the small kernel takes, more layers than one batched launch takes, ragged batches
+def _pass(sizes, m):
+    """Random weights, the library's forward and backward over them; everything it wrote."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(m + len(sizes))
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    k, n = sizes[:-1], sizes[1:]
+    layers, last = len(n), n[-1]
+    w = [rand(b, a) / a**0.5 for a, b in zip(k, n)]
+    b = [rand(c) for c in n]
+    x, dy = rand(m, k[0]), rand(m, last)
+    pre = [torch.empty(m, c, device="cuda") for c in n[:-1]]
+    act = [torch.empty(m, c, dtype=torch.bfloat16, device="cuda") for c in n[:-1]]
+    out = torch.empty(m, last, device="cuda")
+    dw, db = [torch.empty_like(t) for t in w], [torch.empty_like(t) for t in b]
+    lib, ptr = _lib.library(), surrogate._pointers
+    cn, ck = (C.c_int * layers)(*n), (C.c_int * layers)(*k)
+    size = lib.sp_mlp_training_scratch(layers, m, cn, ck)
+    scratch = torch.empty(size, dtype=torch.uint8, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _lib.check(lib.sp_mlp_training_forward(layers, m, cn, ck, ptr(w), ptr(b), x.data_ptr(), k[0], ptr(pre), ptr(act),
+                                           out.data_ptr(), scratch.data_ptr(), size, status.data_ptr(), None))
+    _lib.check(lib.sp_mlp_training_backward(layers, m, cn, ck, ptr(w), x.data_ptr(), k[0], ptr([*pre, None]), ptr(act),
+                                            dy.data_ptr(), ptr(dw), ptr(db), scratch.data_ptr(), size,
+                                            status.data_ptr(), None))
+    assert int(status.item()) == 0
+    return w, b, x, dy, [*pre, out], act, dw, db
+
+
+# Each layer from the library's own activations, in 64 bits with the operands' BF16 rounding: the
+# FP32 sums' error, 1e-5; a gradient whose last bit turned its rounding to BF16 over in a layer
+# above adds at most that rounding, 2^-9, for each of them
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [1, 63, 65])
+@pytest.mark.parametrize("sizes", [(6, 256), (300, 256), (64, 256, 512), (8, 512, 256), (9, 256, 256),
+                                   (6, *[256] * 12), (6, *[256] * 18)], ids=str)
+def test_training_pass_layers(sizes, m):
+    import torch
+
+    w, b, x, dy, pre, act, dw, db = _pass(sizes, m)
+    half = lambda t: t.bfloat16().double()  # noqa: E731
+    inputs = [x, *act]
+    for i, (wi, bi) in enumerate(zip(w, b)):
+        assert _rel(pre[i], half(inputs[i]) @ half(wi).T + bi.double()) < 1e-5, i
+    for p, a in zip(pre, act):
+        z = p.double()
+        assert _rel(a, z / 2 * torch.erfc(-z / 2**0.5)) < 2**-8
+    g = dy.double()
+    for i in reversed(range(len(w))):
+        if i < len(w) - 1:
+            z = pre[i].double()
+            g = g * (0.5 * torch.erfc(-z / 2**0.5) + z * torch.exp(-0.5 * z * z) / (2 * torch.pi) ** 0.5)
+        bound = 1e-5 + (len(w) - 1 - i) * 2**-9
+        assert _rel(db[i], g.sum(0)) < bound, i
+        assert _rel(dw[i], half(g).T @ half(inputs[i])) < bound, i
+        g = half(g) @ half(w[i])
+
+
+def test_training_pass_refusals():
+    lib = _lib.library()
+    n, k = (C.c_int * 2)(256, 256), (C.c_int * 2)(6, 256)
+    size = lib.sp_mlp_training_scratch(2, 5, n, k)
+    some = (C.c_void_p * 2)(256, 256)  # never read: every call is refused first
+    forward = lambda layers, m, n, k, size: lib.sp_mlp_training_forward(  # noqa: E731
+        layers, m, n, k, some, some, 256, 6, some, some, 256, 256, size, 256, None)
+    backward = lambda layers, m, n, k, size: lib.sp_mlp_training_backward(  # noqa: E731
+        layers, m, n, k, some, 256, 6, some, some, 256, some, some, 256, size, 256, None)
+    apart = (C.c_int * 2)(6, 128)
+    many = (C.c_int * 65)(*[256] * 65)
+    assert size > 0 and lib.sp_mlp_training_scratch(64, 5, many, many) > 0
+    argument = 1  # SP_ERR_ARGUMENT
+    for call in (forward, backward):
+        assert call(2, 0, n, k, size) == call(0, 5, n, k, size) == call(2, 5, n, apart, size) == argument
+        assert call(65, 5, many, many, 1 << 40) == argument
+        assert call(2, 5, n, k, 0) == argument
+    assert backward(2, 5, n, k, size - 1) == argument  # the larger of the two
