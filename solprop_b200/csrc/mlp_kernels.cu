@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(1024) k_first_layer_backward(const float* __re
   }
 }
 
-// dY = 2 (Y - T) / (M N); per-row partial losses, summed by k_loss_total in row order
+// dY = 2 (Y - T) / (M N); per-row partial losses, summed by k_loss_total
 __global__ void k_mse(const float* Y, const float* T, int M, int N, float* dY, float* row_loss) {
   const int m = blockIdx.x;
   __shared__ float part[256];
@@ -280,7 +280,8 @@ __global__ void k_mse(const float* Y, const float* T, int M, int N, float* dY, f
   if (threadIdx.x == 0) row_loss[m] = part[0];
 }
 
-__global__ void k_loss_total(const float* row_loss, int M, int N, float* loss) {  // one warp
+// one warp: lane l sums rows l, l + 32, ... in order, then the lanes as a tree, in FP64
+__global__ void k_loss_total(const float* row_loss, int M, int N, float* loss) {
   double s = 0.0;
   for (int m = threadIdx.x; m < M; m += 32) s += row_loss[m];
 #pragma unroll

@@ -307,39 +307,16 @@ __global__ void k_to_bf16(const float* src, int ld_src, int rows, int cols, __nv
   }
 }
 
-// dst[c][r] = BF16(src[r][c]) for r < rows, zero for rows <= r < rows_pad (32 x 32 tiles
-// through shared memory, both sides coalesced)
-template <class T>
-__global__ void k_transpose_bf16(const T* src, int ld_src, int rows, int cols, __nv_bfloat16* dst, int ld_dst,
-                                 int rows_pad) {
-  __shared__ float tile[32][33];
-  const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int r = r0 + i, c = c0 + threadIdx.x;
-    float v = 0.0f;
-    if (r < rows && c < cols) {
-      if constexpr (sizeof(T) == 4) v = src[(size_t)r * ld_src + c];
-      else v = __bfloat162float(src[(size_t)r * ld_src + c]);
-    }
-    tile[i][threadIdx.x] = v;
-  }
-  __syncthreads();
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int c = c0 + i, r = r0 + threadIdx.x;
-    if (c < cols && r < rows_pad) dst[(size_t)c * ld_dst + r] = __float2bfloat16_rn(tile[threadIdx.x][i]);
-  }
-}
-
 // Several matrices in one launch: of each FP32 (or BF16) rows x cols matrix a BF16 copy with rows
-// of cols_out (zero-padded) and / or a BF16 transpose with rows of rows_pad (zero-padded).  Block
-// b takes the 32 x 32 tile b - first[q] of matrix q; the source is read once.
+// of cols_out (zero-padded) and / or a BF16 transpose with rows of rows_pad (zero-padded), ld_t
+// apart.  Block b takes the 32 x 32 tile b - first[q] of matrix q; the source is read once.
 constexpr int kMaxConversions = 8;
 struct ConvertBatch {
   const void* src[kMaxConversions];
   __nv_bfloat16* copy[kMaxConversions];
   __nv_bfloat16* transpose[kMaxConversions];
   int rows[kMaxConversions], cols[kMaxConversions], ld[kMaxConversions];
-  int cols_out[kMaxConversions], rows_pad[kMaxConversions], tiles_c[kMaxConversions];
+  int cols_out[kMaxConversions], rows_pad[kMaxConversions], ld_t[kMaxConversions], tiles_c[kMaxConversions];
   int first[kMaxConversions + 1];
   int count;
 };
@@ -369,7 +346,7 @@ __global__ void __launch_bounds__(256) k_convert_bf16(const __grid_constant__ Co
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int c = c0 + ty + 8 * i, r = r0 + tx;
-    if (c < p.cols[q] && r < p.rows_pad[q]) transpose[(size_t)c * p.rows_pad[q] + r] = tile[tx][ty + 8 * i];
+    if (c < p.cols[q] && r < p.rows_pad[q]) transpose[(size_t)c * p.ld_t[q] + r] = tile[tx][ty + 8 * i];
   }
 }
 
@@ -488,14 +465,19 @@ sp_status sp_mlp_transpose_bf16(const void* src, int src_bf16, int ld_src, int r
                                 int ld_dst, int rows_pad, void* stream) {
   if (!src || !dst || rows < 0 || cols < 0 || rows_pad < rows || ld_dst < rows_pad) return SP_ERR_ARGUMENT;
   if (!rows_pad || !cols) return SP_OK;
-  const dim3 grid((cols + 31) / 32, (rows_pad + 31) / 32), block(32, 8);
-  if (src_bf16)
-    sp::k_transpose_bf16<__nv_bfloat16><<<grid, block, 0, (cudaStream_t)stream>>>(
-        static_cast<const __nv_bfloat16*>(src), ld_src, rows, cols, static_cast<__nv_bfloat16*>(dst), ld_dst,
-        rows_pad);
-  else
-    sp::k_transpose_bf16<float><<<grid, block, 0, (cudaStream_t)stream>>>(
-        static_cast<const float*>(src), ld_src, rows, cols, static_cast<__nv_bfloat16*>(dst), ld_dst, rows_pad);
+  sp::ConvertBatch p{};
+  p.count = 1;
+  p.src[0] = src;
+  p.transpose[0] = static_cast<__nv_bfloat16*>(dst);
+  p.rows[0] = rows;
+  p.cols[0] = cols;
+  p.ld[0] = ld_src;
+  p.rows_pad[0] = rows_pad;
+  p.ld_t[0] = ld_dst;
+  p.tiles_c[0] = (cols + 31) / 32;
+  p.first[1] = p.tiles_c[0] * ((rows_pad + 31) / 32);
+  if (src_bf16) sp::k_convert_bf16<__nv_bfloat16><<<p.first[1], 256, 0, (cudaStream_t)stream>>>(p);
+  else sp::k_convert_bf16<float><<<p.first[1], 256, 0, (cudaStream_t)stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? SP_OK : SP_ERR_CUDA;
 }
 
@@ -518,7 +500,7 @@ sp_status sp_mlp_convert_batch(int count, int src_bf16, const void* const* src, 
     p.cols[q] = cols[q];
     p.ld[q] = ld[q];
     p.cols_out[q] = cols_out[q];
-    p.rows_pad[q] = rows_pad[q];
+    p.rows_pad[q] = p.ld_t[q] = rows_pad[q];
     const int r = transpose[q] ? rows_pad[q] : rows[q], c = copy[q] ? cols_out[q] : cols[q];
     p.tiles_c[q] = (c + 31) / 32;
     p.first[q + 1] = p.first[q] + p.tiles_c[q] * ((r + 31) / 32);

@@ -64,6 +64,14 @@ def test_batched_conversion_and_adam():
         r, k = x.shape
         assert torch.equal(c[:, :k], x.bfloat16()) and not c[:, k:].any()
         assert torch.equal(t[:, :r], x.bfloat16().T) and not t[:, r:].any()
+    for x, pad in zip(xs, pads):  # one matrix on its own, rows of the transpose further apart
+        for src in (x, x.bfloat16()):
+            t = new(x.shape[1], pad + 3)
+            _lib.check(_lib.library().sp_mlp_transpose_bf16(src.data_ptr(), int(src is not x), x.shape[1], *x.shape,
+                                                            t.data_ptr(), pad + 3, pad, None))
+            assert torch.equal(t[:, :x.shape[0]], x.bfloat16().T) and not t[:, x.shape[0]:pad].any()
+            assert t[:, pad:].isnan().all()
+            assert torch.equal(surrogate.transpose_bf16(src, pad), t[:, :pad])
     net, one = surrogate.Perceptron(7), surrogate.Perceptron(7)
     grads = [torch.randn(p.shape, device="cuda", generator=g) for p in net.params]
     net.adam(grads, 1e-3)
