@@ -292,10 +292,11 @@ struct sp_workspace {
   DevBuf<long long> crop;
   DevBuf<int> fine_to_coarse, rows, chain_flags;
   DevBuf<unsigned long long> ticket;  // the response column's tile counter
-  DevBuf<double2> env_twiddles;       // envelope route: exp(-2 pi i m / (2 n_to)), m < n_to
+  // exp(-2 pi i m / (2 n_to)), m < n_to: field-grid Raman, the envelope products' long rows
+  DevBuf<double2> env_twiddles;
   DevBuf<double> raman_undamped, raman_weights;
   DevBuf<double> stat_power, stat_out, stat_weight;  // plane statistics, on first use
-  DevBuf<double2> raman_spectrum;  // field-grid Raman: the damped kernel's spectrum (n_to + 1)
+  DevBuf<double2> raman_spectrum;  // ... and the damped kernels' spectra (raman_kernels, n_to + 1)
   DevBuf<int> raman_scale;         // the envelope products' mixed form: the spectra's powers of two
   // the envelope products' nodes: the spectra and twiddles in the register transform's order
   DevBuf<double2> raman_table, row_outer, row_inner;
@@ -705,7 +706,8 @@ static EnvModalArgsT<R> env_modal_args(const sp_workspace* ws, const double2* la
   ea.fine_to_coarse = ws->fine_to_coarse.p;
   ea.row_outer = ws->row_outer.p;
   ea.row_inner = ws->row_inner.p;
-  ea.raman_spectrum = d.raman_enabled ? ws->raman_spectrum.p : nullptr;
+  ea.raman = d.raman_enabled;
+  ea.raman_spectrum = ws->raman_spectrum.p;
   ea.n_cols = P.n_cols;
   ea.n_omega = d.n_omega;
   ea.n_to = d.n_to;
@@ -1063,10 +1065,12 @@ static void build_workspace(sp_workspace* ws) {
   ws->norm_arrivals.alloc(1);
   ws->norm_arrivals.zero(s);
   ws->launches = 5;
-  if (ws->gemm && d.grid_kind == 1) {  // inverse, synthesis, (long rows: Raman spectrum, table,) nodes, projection, reduction,
-    const bool long_rows = d.n_to > kMaxEnvelopeRowF64;  // the spectrum (and the mixed form's table) on their own
-    ws->launches = 6 + (d.raman_enabled && long_rows ? ws->precision == SP_PRECISION_MIXED ? 2 : 1 : 0) + (ws->precision == SP_PRECISION_MIXED ? 1 : 0);  // forward,
-                                                                  // output; the mixed form's split pass
+  // the envelope products' rows that take the long FP64 transforms (the mixed form's inverse alone)
+  const bool long_rows = d.grid_kind == 1 && ws->gemm && d.n_to > kMaxEnvelopeRowF64;
+  if (ws->gemm && d.grid_kind == 1) {
+    const int mixed = ws->precision == SP_PRECISION_MIXED;
+    ws->launches = 6 + mixed;  // inverse, synthesis (split, product), nodes, projection, reduction, forward, output
+    if (d.raman_enabled && long_rows) ws->launches += 1 + mixed;  // the kernels' spectra, their FP32 table
   } else if (ws->gemm) {  // inverse, synthesis, column, one projection per stream, forward, output
     const int synthesis = ws->precision == SP_PRECISION_MIXED ? 2 : 1;  // (split,) product
     const int streams = d.plasma_enabled ? 3 : 1;  // each: product, reduction of the K splits
@@ -1074,10 +1078,10 @@ static void build_workspace(sp_workspace* ws) {
   }
   if (ws->precision == SP_PRECISION_MIXED) build_mixed(ws, tw, rc, taps);
   if (!tw2.empty()) {
-    ws->env_twiddles.upload(tw2.data(), tw2.size(), s);
+    if (d.grid_kind == 0 || long_rows) ws->env_twiddles.upload(tw2.data(), tw2.size(), s);
     if (d.raman_enabled) ws->raman_undamped.upload(P.raman_undamped.data(), P.raman_undamped.size(), s);
     if (!P.raman_weights.empty()) ws->raman_weights.upload(P.raman_weights.data(), P.raman_weights.size(), s);
-    if (d.raman_enabled && (d.grid_kind == 0 || ws->gemm))
+    if (d.raman_enabled && (d.grid_kind == 0 || long_rows))
       ws->raman_spectrum.alloc((size_t)P.raman_kernels * (d.n_to + 1));
     if (d.grid_kind == 1) {
       // the register transform's tables (FP64 rows above kMaxEnvelopeRowF64 take the long form)
@@ -1104,7 +1108,7 @@ static void build_workspace(sp_workspace* ws) {
         ws->raman_scale.alloc(2);
       }
     }
-    if (d.grid_kind == 1 && ws->gemm && d.n_to > kMaxEnvelopeRowF64) {
+    if (long_rows) {
       // rows of FP64 too long for one CTA: the inverse transforms' (every column), and in the
       // FP64 form the nodes' and the forward transforms'
       const size_t rows = ws->precision == SP_PRECISION_MIXED ? (size_t)P.n_cols

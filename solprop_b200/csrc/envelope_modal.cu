@@ -16,9 +16,9 @@
 //   k_env_forward  one CTA per modal column: fft of the projected row, cropped
 //
 // Every transform is the register FFT of fft_regs.cuh (FP64 rows of 16 384 samples: the halves
-// of fft_long.cuh over the table exp(-2 pi i m / (2 n_to)), m < n_to).  The inverse transform and the modal field are FP64
-// in both forms; the Kerr cubic, the Raman convolutions and the forward transform run in the
-// form's type R (FP32 in the mixed form).
+// of fft_long.cuh over the table exp(-2 pi i m / (2 n_to)), m < n_to).  The inverse transform and
+// the modal field are FP64 in both forms; the Kerr cubic, the Raman convolutions and the forward
+// transform run in the form's type R (FP32 in the mixed form).
 #include <algorithm>
 #include <type_traits>
 
@@ -36,10 +36,10 @@ constexpr int kEnvThreads = 1024;
 
 // A column's (or kernel's) transform is one CTA's chain of passes, run once: what bounds it is
 // latency, the instructions' own fetch included, so its threads hold 16 points where the three
-// passes allow it (fft_regs.cuh).  30 columns of 4 096 and two
-// Raman kernels, ncu: the inverse and the kernels' spectra 32.6 + 28.6 us with shared-memory
-// radix-4 transforms in launches of their own -> 32.4 us, the FP32 forward 14.7 -> 13.4 (with
-// 32 points per thread 28.6); FP64 columns of 8 192: 66 + 46 -> 57 us, the forward 34 us.
+// passes allow it (fft_regs.cuh).  30 columns of 4 096 and two Raman kernels, ncu: the inverse and
+// the kernels' spectra 32.6 + 28.6 us with shared-memory radix-4 transforms in launches of their
+// own -> 32.4 us, the FP32 forward 14.7 -> 13.4 (with 32 points per thread 28.6); FP64 columns of
+// 8 192: 66 + 46 -> 57 us, the forward 34 us.
 
 // The Raman kernels' spectra in k_env_pairs' order (rows of up to 8 192; longer ones take
 // k_raman_kernel and k_raman_table): one CTA per kernel and half p transforms the damped
@@ -540,16 +540,11 @@ __global__ void __launch_bounds__(kNodeThreads, 1) k_env_nodes_long(EnvModalArgs
   const double2* Ey = Ex + (nc == 2 ? n : 0);
   double2* Px = reinterpret_cast<double2*>(a.node_streams) + (size_t)node * nc * n;
   double2* Py = Px + (nc == 2 ? n : 0);
-  const bool raman = a.raman_spectrum != nullptr;
-  const int drives = !raman ? 0 : (nc == 2 && a.raman_kernels == 2 ? 3 : 1);
+  const int drives = nc == 2 && a.raman_kernels == 2 ? 3 : 1;
   const double factor = a.kerr ? a.kerr_coefficient * st.kerr_density : 0.0;
   const double self = a.kerr_self, conj = a.kerr_conjugate;
   const double raman_scale = kEps0 * (a.raman_mixture ? 1.0 : st.raman_density);
   const double inv_n = 1.0 / (double)n;
-  if (drives == 0) {
-    for (int t = threadIdx.x; t < n; t += blockDim.x) node_sample<double>(a, Ex, Ey, Px, Py, t, 0.0, 0, nc, factor, self, conj);
-    return;
-  }
   for (int dr = 0; dr < drives; ++dr) {
     // the drive on [0, n), zero on [n, 2n), packed b[m] = d(2m) + i d(2m + 1), transformed
     long_forward(
@@ -692,7 +687,7 @@ cudaError_t launch_env_inverse(const EnvModalArgsT<R>& a, const RamanArgs* raman
 
 template <class R>
 cudaError_t launch_env_nodes(const EnvModalArgsT<R>& a, int n_nodes, cudaStream_t s) {
-  if (!a.raman_spectrum) {
+  if (!a.raman) {
     const size_t total = (size_t)n_nodes * a.n_to;
     k_env_kerr<R><<<(unsigned)std::min<size_t>((total + 255) / 256, 148 * 16), 256, 0, s>>>(a, n_nodes);
     return cudaGetLastError();

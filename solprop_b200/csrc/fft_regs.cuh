@@ -111,7 +111,7 @@ struct Row {
   static constexpr int kLogV = LOGV, V = 1 << kLogV;
   static constexpr int N = 1 << LOGN, T = N / V, M = T, G = M / V;
   static constexpr int kLogG = LOGN - 2 * kLogV;
-  static_assert(kLogG >= 0 && G <= V && G <= 32 && T >= 32, "N = V V G with G threads of a warp per row");
+  static_assert(kLogG >= 1 && G <= V && G <= 32 && T >= 32, "N = V V G with G threads of a warp per row");
   static constexpr int kPitch = M + G;                 // a padded row (one element per V)
   static constexpr size_t kPlane = (size_t)V * kPitch;  // reals of the exchange plane
   // offset of row point m = j + G r beside j < G (the padding (j + G r) / V does not depend on j)
@@ -144,35 +144,32 @@ struct Row {
       x[r].y = row[j + strided(r)];
     }
     dft_dif<kLogV>(x);
-    if constexpr (G > 1) {
-      const C* const tw_row = inner + j;
+    const C* const tw_row = inner + j;
 #pragma unroll
-      for (int i = 0; i < V; ++i)
-        if (i > 0) x[i] = cmul(x[i], tw_row[rev(i, kLogV) * G]);
-      __syncwarp();  // the row's other threads have read it
+    for (int i = 0; i < V; ++i)
+      if (i > 0) x[i] = cmul(x[i], tw_row[rev(i, kLogV) * G]);
+    __syncwarp();  // the row's other threads have read it
 #pragma unroll
-      for (int i = 0; i < V; ++i) row[j + strided(rev(i, kLogV))] = x[i].x;
-      __syncwarp();
+    for (int i = 0; i < V; ++i) row[j + strided(rev(i, kLogV))] = x[i].x;
+    __syncwarp();
 #pragma unroll
-      for (int e = 0; e < V; ++e) re[e] = row[j * (V + 1) + e];
-      __syncwarp();
+    for (int e = 0; e < V; ++e) re[e] = row[j * (V + 1) + e];
+    __syncwarp();
 #pragma unroll
-      for (int i = 0; i < V; ++i) row[j + strided(rev(i, kLogV))] = x[i].y;
-      __syncwarp();
+    for (int i = 0; i < V; ++i) row[j + strided(rev(i, kLogV))] = x[i].y;
+    __syncwarp();
 #pragma unroll
-      for (int e = 0; e < V; ++e) {
-        x[e].x = re[e];
-        x[e].y = row[j * (V + 1) + e];
-      }
-#pragma unroll
-      for (int s = 0; s < V; s += G) dft_dif<kLogG>(x + s);
+    for (int e = 0; e < V; ++e) {
+      x[e].x = re[e];
+      x[e].y = row[j * (V + 1) + e];
     }
+#pragma unroll
+    for (int s = 0; s < V; s += G) dft_dif<kLogG>(x + s);
   }
 
   // the bin of register e of pass 3: set e / G (g = j V / G + e / G), DFT output h
   static __host__ __device__ constexpr int bin(int t, int e) {
-    if constexpr (G == 1) return t + V * rev(e, kLogV);
-    else return t / G + V * ((t % G) * (V / G) + e / G + V * rev(e % G, kLogG));
+    return t / G + V * ((t % G) * (V / G) + e / G + V * rev(e % G, kLogG));
   }
 
   // the inverse (unnormalised) of forward: points of pass 3 -> natural x[t + r T]
@@ -182,29 +179,27 @@ struct Row {
     R* const column = plane + t + (t >> kLogV);
     R* const row = plane + (t / G) * kPitch;
     R re[V];
-    if constexpr (G > 1) {
 #pragma unroll
-      for (int s = 0; s < V; s += G) dft_dit_inverse<kLogG>(x + s);
-      __syncwarp();
+    for (int s = 0; s < V; s += G) dft_dit_inverse<kLogG>(x + s);
+    __syncwarp();
 #pragma unroll
-      for (int e = 0; e < V; ++e) row[j * (V + 1) + e] = x[e].x;
-      __syncwarp();
+    for (int e = 0; e < V; ++e) row[j * (V + 1) + e] = x[e].x;
+    __syncwarp();
 #pragma unroll
-      for (int i = 0; i < V; ++i) re[i] = row[j + strided(rev(i, kLogV))];
-      __syncwarp();
+    for (int i = 0; i < V; ++i) re[i] = row[j + strided(rev(i, kLogV))];
+    __syncwarp();
 #pragma unroll
-      for (int e = 0; e < V; ++e) row[j * (V + 1) + e] = x[e].y;
-      __syncwarp();
+    for (int e = 0; e < V; ++e) row[j * (V + 1) + e] = x[e].y;
+    __syncwarp();
 #pragma unroll
-      for (int i = 0; i < V; ++i) {
-        x[i].x = re[i];
-        x[i].y = row[j + strided(rev(i, kLogV))];
-      }
-      const C* const tw_row = inner + j;
-#pragma unroll
-      for (int i = 0; i < V; ++i)
-        if (i > 0) x[i] = cmul(x[i], cconj(tw_row[rev(i, kLogV) * G]));
+    for (int i = 0; i < V; ++i) {
+      x[i].x = re[i];
+      x[i].y = row[j + strided(rev(i, kLogV))];
     }
+    const C* const tw_row = inner + j;
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+      if (i > 0) x[i] = cmul(x[i], cconj(tw_row[rev(i, kLogV) * G]));
     dft_dit_inverse<kLogV>(x);
     __syncwarp();  // the row's other threads have read it
 #pragma unroll

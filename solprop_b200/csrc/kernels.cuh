@@ -228,8 +228,9 @@ struct RamanArgs {
   // kernels formed (1: the trace; 2: trace and traceless, spectra (2, n_to + 1)); null: scalar
   const double* tensor_weights;
   int n_kernels;
-  // the mixed form's envelope products: the power of two 2^scale[kernel] that brings each
-  // spectrum's largest bin near one, for its FP32 table (else null)
+  // the mixed form's envelope products: the power of two 2^scale[kernel] that brings each spectrum
+  // near one for its FP32 table (rows above kMaxEnvelopeRowF64: its largest bin, else the bins'
+  // bound, the kernel's sum of magnitudes, into [1, 2)); null without
   int* scale;
   double2* scratch;  // rows above kMaxEnvelopeRowF64: 1.5 n_to complex per kernel
 };
@@ -263,7 +264,7 @@ struct EnvModalArgsT {
   const StageScalarsDev* stage;
   const double2* lab;             // (n_cols, n_omega)
   const long long* crop;          // (n_omega): coarse bin -> fine bin
-  const double2* twiddles;        // exp(-2 pi i m / (2 n_to)), m < n_to
+  const double2* twiddles;        // exp(-2 pi i m / (2 n_to)), m < n_to: rows above kMaxEnvelopeRowF64
   const double* t_window;         // (n_to)
   const double* alpha;            // the in-stage absorber's rate (n_to), or null
   double* modal_t;                // (n_cols, 2 n_to): a(t)
@@ -272,7 +273,7 @@ struct EnvModalArgsT {
   const R* projected;             // (n_cols, 2 n_to): sum W P / tau
   cplx<R>* spectra;               // (4, n_cols, n_omega): P, -, -, absorber
   double2* scratch;               // FP64 rows above kMaxEnvelopeRowF64: 1.5 n_to per row
-  const double2* raman_spectrum;  // (raman_kernels, n_to + 1), or null without Raman
+  const double2* raman_spectrum;  // (raman_kernels, n_to + 1): rows above kMaxEnvelopeRowF64
   const int* raman_scale;         // the mixed form: the powers of two inside raman_table
   // the register transform (fft_regs.cuh): the nodes' Raman spectra in its bin order,
   // (raman_kernels, 2 n_to), its two twiddle tables
@@ -282,7 +283,7 @@ struct EnvModalArgsT {
   const double2* row_outer;       // the same in FP64 (rows of up to kMaxEnvelopeRowF64)
   const double2* row_inner;
   const int* fine_to_coarse;      // (n_to): the coarse bin of a fine one, or -1
-  int n_cols, n_omega, n_to, log_n_to, kerr, raman_mixture;
+  int n_cols, n_omega, n_to, log_n_to, kerr, raman, raman_mixture;
   int n_components;               // field components per node (1, or 2: rows x, y)
   int raman_kernels;              // two components: 1 (trace) or 2 (trace, traceless)
   double kerr_coefficient, kerr_self, kerr_conjugate;
