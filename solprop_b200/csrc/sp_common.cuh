@@ -63,16 +63,22 @@ template <> __host__ __device__ __forceinline__ float2 to_c<float2>(double2 v) {
 __host__ __device__ __forceinline__ double2 to_d2(double2 v) { return v; }
 __host__ __device__ __forceinline__ double2 to_d2(float2 v) { return make_double2(v.x, v.y); }
 
-// ---- a single run's chain of short kernels: each is launched while the one before it runs
-// (programmatic dependent launch) and waits here, before its first access to global memory,
-// for that one's end; and it lets the next be launched at once.  Every kernel of the chain
-// waits, so each sees the writes of all before it.  A kernel launched in the ordinary way
-// passes straight through.  It saves a launch's latency per kernel, about 1 us of 5.
+// ---- a single run's chain of short kernels: each is launched as the last CTAs of the one before it
+// end (programmatic dependent launch) and waits here, before its first access to global memory,
+// for that one's end and its writes.  Every kernel of the chain waits, so each sees the writes of
+// all before it.  A kernel launched in the ordinary way passes straight through.  It saves a
+// launch's latency per kernel, about 1 us of 5.
+// No kernel triggers the next one earlier (griddepcontrol.launch_dependents): CTAs that wait hold
+// their place on an SM, the next kernels' are packed onto the first SMs that free up, and other
+// streams find none.  With the trigger ahead of the wait, the whole chain resident at once, 24
+// attempts of eight mixed modes, rows of 4 096, took 2.28 ms (2.02 in ordinary launches, 1.75
+// now), and evaluations of four mixed modes, rows of 32 768, of three workspaces in turn 48.2 us
+// each (46.6; 40.3).  Over 128 sizes the chain was 0.89 to 1.44 times as fast as ordinary
+// launches with that trigger, and is 1.06 to 1.55 times as fast without.
 // Such a kernel runs beside the one that writes its inputs, and non-coherent loads are not ordered
 // after the wait: __ldg and const __restrict__ are for tables written at workspace creation alone,
 // what an earlier kernel of the chain wrote is read by plain loads or __ldcg.
 __device__ __forceinline__ void await_previous_kernel() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 // launches a kernel that begins with await_previous_kernel, in clusters of `cluster` CTAs along x

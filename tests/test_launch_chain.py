@@ -33,3 +33,9 @@ def test_chained_kernels_read_the_chain_coherently():
     for path in CHAINED:
         for name, parameters, first in _kernels(path.read_text()):
             assert first != "await_previous_kernel();" or "__restrict__" not in parameters, name
+
+
+def test_no_kernel_lets_the_next_in_before_it_ends():
+    """A trigger ahead of a kernel's work makes the whole chain resident, waiting on SMs that other
+    kernels and streams need: runs of rows of 4 096 were up to a tenth slower than unchained."""
+    assert not [p.name for p in CSRC.glob("*.cu*") if re.search(r'"griddepcontrol.launch_dependents', p.read_text())]
