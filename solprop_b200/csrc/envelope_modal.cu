@@ -290,7 +290,7 @@ __device__ __forceinline__ void balance(cplx<R> (&x)[Row::V], WarpGauge<R>* part
   }
 }
 
-// The nodes' responses with Raman, one CTA per two nodes A and B.  A convolution with a real
+// The nodes' responses with Raman, one CTA per two nodes A and B (or one node).  A convolution with a real
 // kernel takes two real drives as one complex row: the trace drives of A and B together
 // (drive |a|^2 / 2, or |a_x|^2 / 2 + |a_y|^2 / 2 of two field components), then, where the
 // tensor response has a traceless kernel, each node's difference |a_x|^2 / 2 - |a_y|^2 / 2
@@ -308,7 +308,7 @@ __device__ __forceinline__ void balance(cplx<R> (&x)[Row::V], WarpGauge<R>* part
 // 8 192, FP64: 2.78 -> 1.0 ms.
 template <class R, int LOGN>
 __global__ void __launch_bounds__(regs::Row<cplx<R>, LOGN>::T, pairs_resident<R, LOGN>())
-    k_env_pairs(EnvModalArgsT<R> a, int n_nodes) {
+    k_env_pairs(EnvModalArgsT<R> a, int n_nodes, int per_cta) {
   using C = cplx<R>;
   using Row = regs::Row<C, LOGN>;
   constexpr int n = Row::N, T = Row::T, V = Row::V;
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(regs::Row<cplx<R>, LOGN>::T, pairs_resident<R,
   C* stash = reinterpret_cast<C*>(ep_raw);
   R* plane = reinterpret_cast<R*>(stash + n);
   const int nc = a.n_components, t0 = threadIdx.x;
-  const int first = 2 * blockIdx.x, count = min(2, n_nodes - first);
+  const int first = per_cta * blockIdx.x, count = min(per_cta, n_nodes - first);
   const StageScalarsDev& st = *a.stage;
   const double factor = a.kerr ? a.kerr_coefficient * st.kerr_density : 0.0;
   const double density = kEps0 * (a.raman_mixture ? 1.0 : st.raman_density);  // a mixture's are inside
@@ -697,9 +697,14 @@ cudaError_t launch_env_nodes(const EnvModalArgsT<R>& a, int n_nodes, cudaStream_
       k_env_nodes_long<<<n_nodes, kNodeThreads, (size_t)a.n_to / 2 * sizeof(double2), s>>>(a);
     return cudaGetLastError();
   }
+  // Two nodes a CTA take three convolutions where one takes two (the tensor response): with no more
+  // nodes than SMs a CTA each is the shorter chain.  49 nodes, FP64 rows of 1 024: 40 -> 27 us (a run:
+  // 1.73 -> 1.55 ms); 169 nodes, more than SMs, keep two a CTA: three convolutions for four.
+  const int per_cta = a.n_components == 2 && a.raman_kernels == 2 && n_nodes <= 148 ? 1 : 2;
   return with_row<R>(a.log_n_to, [&](auto log) {
     constexpr int LOGN = decltype(log)::value;
-    k_env_pairs<R, LOGN><<<(n_nodes + 1) / 2, regs::Row<cplx<R>, LOGN>::T, pairs_smem<R, LOGN>(), s>>>(a, n_nodes);
+    k_env_pairs<R, LOGN><<<(n_nodes + per_cta - 1) / per_cta, regs::Row<cplx<R>, LOGN>::T, pairs_smem<R, LOGN>(), s>>>(
+        a, n_nodes, per_cta);
     return cudaGetLastError();
   });
 }
