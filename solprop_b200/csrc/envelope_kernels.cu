@@ -37,7 +37,7 @@ constexpr int kRanks = 4;
 }  // namespace
 
 template <int LOGN>
-using EnvelopeRow = regs::Row<double2, LOGN, 4>;
+using EnvelopeRow = regs::Row<double2, LOGN>;
 template <int LOGN>
 constexpr size_t envelope_smem() {
   return EnvelopeRow<LOGN>::N * sizeof(double2) + EnvelopeRow<LOGN>::kPlane * sizeof(double);

@@ -221,11 +221,12 @@ __device__ __forceinline__ void node_output(const EnvModalArgsT<R>& a, int nc, d
   }
 }
 
-// resident CTAs: the rows fill the registers of an SM (V points of 8 or 16 bytes and as much again)
+// resident CTAs: the rows fill the registers of an SM (V points of 8 or 16 bytes and as much again,
+// 64 or 128 registers a thread at least)
 template <class R, int LOGN>
 constexpr int pairs_resident() {
   using Row = regs::Row<cplx<R>, LOGN>;
-  return (sizeof(R) == 4 ? 16384 : 8192) / Row::V / Row::T;
+  return (sizeof(R) == 4 ? 16384 : 8192) / (Row::V < 16 ? 16 : Row::V) / Row::T;
 }
 
 // The second drive of a complex row is brought to the first one's norm by a power of two: a
@@ -697,10 +698,10 @@ cudaError_t launch_env_nodes(const EnvModalArgsT<R>& a, int n_nodes, cudaStream_
       k_env_nodes_long<<<n_nodes, kNodeThreads, (size_t)a.n_to / 2 * sizeof(double2), s>>>(a);
     return cudaGetLastError();
   }
-  // Two nodes a CTA take three convolutions where one takes two (the tensor response): with no more
-  // nodes than SMs a CTA each is the shorter chain.  49 nodes, FP64 rows of 1 024: 40 -> 27 us (a run:
-  // 1.73 -> 1.55 ms); 169 nodes, more than SMs, keep two a CTA: three convolutions for four.
-  const int per_cta = a.n_components == 2 && a.raman_kernels == 2 && n_nodes <= 148 ? 1 : 2;
+  // Two nodes a CTA take three convolutions of the tensor response where one takes two, and twice the
+  // outputs: with no more nodes than SMs a CTA each is the shorter chain.  49 nodes, FP64 rows of
+  // 1 024: 40 -> 27 us; 64 of one component: 27 -> 18 us.  Of 169, more than SMs, two a CTA.
+  const int per_cta = n_nodes <= 148 ? 1 : 2;
   return with_row<R>(a.log_n_to, [&](auto log) {
     constexpr int LOGN = decltype(log)::value;
     k_env_pairs<R, LOGN><<<(n_nodes + per_cta - 1) / per_cta, regs::Row<cplx<R>, LOGN>::T, pairs_smem<R, LOGN>(), s>>>(

@@ -1,5 +1,5 @@
 // A complex FFT of N = 2^LOGN points held in the registers of one CTA, for the envelope
-// grid: N / V threads of V points each (V = 32, or 16 for short rows).
+// grid: N / V threads of V points each (V = 32; 16 or 8 for short rows).
 //
 // The factorisation is N = V x V x G, G = N / V^2 <= 16, decimation in frequency:
 //   pass 1  thread t holds x[t + r T], r < V (T = N / V threads): a V-point DFT over r, the
@@ -101,9 +101,10 @@ __device__ __forceinline__ void dft_dit_inverse(C* x) {
 // may keep in registers from the forward transform to the inverse, which reads the same
 // twiddles, and the row is spilled to make room for them.
 
-// 16 points a thread where the three passes allow it (N <= 4 096): the same exchanges as with 32,
-// half the unrolled code and twice the warps
-constexpr int default_log_v(int log_n) { return log_n <= 12 ? 4 : 5; }
+// 16 points a thread where the three passes allow it (N <= 4 096), 8 for N = 512: the same exchanges
+// as with 32, half the unrolled code and twice the warps.  512 with 16, one warp a row: the inverse
+// and the Raman spectrum of 15 FP64 columns 18.9 us, the forward 8.6; with 8 points 9.9 and 5.2
+constexpr int default_log_v(int log_n) { return log_n <= 9 ? 3 : log_n <= 12 ? 4 : 5; }
 
 template <class C, int LOGN, int LOGV = default_log_v(LOGN)>
 struct Row {

@@ -170,7 +170,7 @@ struct OutputArgs {
 };
 
 // The envelope route (envelope_kernels.cu): one modal column on one node, one cluster.
-constexpr int kMaxEnvelopeSamples = 4096;   // rows of 256 threads of 16 points
+constexpr int kMaxEnvelopeSamples = 4096;   // rows of at most 256 threads of 16 points
 constexpr int kMaxEnvelopeProducts = 16384;  // the products route's rows
 constexpr int kMaxEnvelopeRowF64 = 8192;     // an FP64 row in one CTA's shared memory; longer
                                              // FP64 rows take two halves and a global scratch
@@ -178,7 +178,7 @@ struct EnvelopeArgs {
   const StageScalarsDev* stage;
   const double2* lab;            // (n_omega)
   const int* fine_to_coarse;     // (n_to): the coarse bin of a fine one, or -1
-  const double2* outer;          // the register transform's tables (fft_regs.cuh, 16 points a thread)
+  const double2* outer;          // the register transform's tables (fft_regs.cuh)
   const double2* inner;
   const double* t_window;        // (n_to)
   const double* raman_undamped;  // (raman_terms, 2 n_to), or null
