@@ -70,7 +70,6 @@ void ensure_configured(int device) {
   CUDA_CHECK(configure_statistics_kernels());
   CUDA_CHECK(configure_modal_gemm());
   CUDA_CHECK(configure_raman_kernels());
-  CUDA_CHECK(configure_env_modal_kernels());
   g_configured[device] = true;
 }
 
@@ -1087,6 +1086,7 @@ static void build_workspace(sp_workspace* ws) {
       // the register transform's tables (FP64 rows above kMaxEnvelopeRowF64 take the long form)
       const bool mixed = ws->precision == SP_PRECISION_MIXED, rows64 = d.n_to <= kMaxEnvelopeRowF64;
       const size_t table = d.raman_enabled && ws->gemm ? (size_t)2 * P.raman_kernels * d.n_to : 0;
+      CUDA_CHECK(ws->gemm ? configure_env_modal_kernels(d.n_to, mixed) : configure_envelope_kernels(d.n_to));
       std::vector<double2> outer, inner;
       row_twiddles(d.n_to, tw2, outer, inner);
       if (rows64) {

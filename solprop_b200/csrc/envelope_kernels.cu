@@ -169,16 +169,12 @@ cudaError_t launch_envelope(const EnvelopeArgs& a, cudaStream_t stream) {
   });
 }
 
-cudaError_t configure_envelope_kernels() {
-  for (int log_n = 9; log_n <= 12; ++log_n) {
-    const cudaError_t e = with_envelope_row(log_n, [](auto log) {
-      constexpr int LOGN = decltype(log)::value;
-      return cudaFuncSetAttribute(k_envelope_source<LOGN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)envelope_smem<LOGN>());
-    });
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+cudaError_t configure_envelope_kernels(int n_to) {
+  return with_envelope_row(31 - __builtin_clz((unsigned)n_to), [](auto log) {
+    constexpr int LOGN = decltype(log)::value;
+    return cudaFuncSetAttribute(k_envelope_source<LOGN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)envelope_smem<LOGN>());
+  });
 }
 
 }  // namespace sp

@@ -612,34 +612,35 @@ static cudaError_t with_row(int log_n, F&& f) {
 template <class C, int LOGN>
 constexpr size_t plane_smem() { return regs::Row<C, LOGN>::kPlane * sizeof(typename regs::Row<C, LOGN>::R); }
 
-cudaError_t configure_env_modal_kernels() {
-  const int row = (int)(kMaxEnvelopeRowF64 * sizeof(double2));  // half a long FP64 row
-  for (const void* k : {(const void*)k_env_inverse_long, (const void*)k_env_inverse_long32,
-                        (const void*)k_env_forward_long, (const void*)k_env_nodes_long}) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, row);
-    if (e != cudaSuccess) return e;
-  }
-  auto configure = [](auto real, int log_n) {
-    using R = decltype(real);
-    return with_row<R>(log_n, [](auto log) {
-      constexpr int LOGN = decltype(log)::value;
-      const auto limit = cudaFuncAttributeMaxDynamicSharedMemorySize;
-      cudaError_t e = cudaFuncSetAttribute(k_env_pairs<R, LOGN>, limit, (int)pairs_smem<R, LOGN>());
+// The kernels of one row length and form: each that is touched is loaded, a third of a millisecond of
+// the first workspace that a process creates (all of them, for any grid: 17 -> 28 ms).
+template <class R>
+static cudaError_t configure_rows(int log_n) {
+  return with_row<R>(log_n, [](auto log) {
+    constexpr int LOGN = decltype(log)::value;
+    const auto limit = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(k_env_pairs<R, LOGN>, limit, (int)pairs_smem<R, LOGN>());
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_env_forward<R, LOGN>, limit, (int)plane_smem<cplx<R>, LOGN>());
+    if constexpr (LOGN <= 13) {
       if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_env_forward<R, LOGN>, limit, (int)plane_smem<cplx<R>, LOGN>());
-      if constexpr (LOGN <= 13) {
-        if (e == cudaSuccess)
-          e = cudaFuncSetAttribute(k_env_inverse<R, LOGN>, limit, (int)plane_smem<double2, LOGN>());
-      }
-      return e;
-    });
-  };
-  for (int log_n = 9; log_n <= 14; ++log_n) {
-    cudaError_t e = configure(0.0f, log_n);
-    if (e == cudaSuccess && log_n <= 13) e = configure(0.0, log_n);
-    if (e != cudaSuccess) return e;
+        e = cudaFuncSetAttribute(k_env_inverse<R, LOGN>, limit, (int)plane_smem<double2, LOGN>());
+    }
+    return e;
+  });
+}
+
+cudaError_t configure_env_modal_kernels(int n_to, bool mixed) {
+  if (n_to > kMaxEnvelopeRowF64) {
+    const int row = (int)(kMaxEnvelopeRowF64 * sizeof(double2));  // half a long FP64 row
+    for (const void* k : {mixed ? (const void*)k_env_inverse_long32 : (const void*)k_env_inverse_long,
+                          (const void*)k_env_forward_long, (const void*)k_env_nodes_long}) {
+      const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, row);
+      if (e != cudaSuccess) return e;
+    }
+    if (!mixed) return cudaSuccess;
   }
-  return cudaSuccess;
+  const int log_n = 31 - __builtin_clz((unsigned)n_to);
+  return mixed ? configure_rows<float>(log_n) : configure_rows<double>(log_n);
 }
 
 void row_twiddles(int n_to, const std::vector<double2>& tw, std::vector<double2>& outer,

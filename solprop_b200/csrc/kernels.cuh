@@ -188,7 +188,7 @@ struct EnvelopeArgs {
   int kerr, raman_terms, n_omega, n_to, log_n_to;
 };
 cudaError_t launch_envelope(const EnvelopeArgs& a, cudaStream_t stream);
-cudaError_t configure_envelope_kernels();
+cudaError_t configure_envelope_kernels(int n_to);
 
 cudaError_t configure_source_kernels();
 
@@ -288,7 +288,7 @@ struct EnvModalArgsT {
   int raman_kernels;              // two components: 1 (trace) or 2 (trace, traceless)
   double kerr_coefficient, kerr_self, kerr_conjugate;
 };
-cudaError_t configure_env_modal_kernels();
+cudaError_t configure_env_modal_kernels(int n_to, bool mixed);
 // with raman (its scale set in the mixed form), also the Raman kernels' spectra into table, the
 // nodes' a.raman_table
 template <class R>
