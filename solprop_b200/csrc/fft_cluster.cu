@@ -164,12 +164,14 @@ __device__ __forceinline__ void forward_cluster_body(const ForwardArgsT<R>& a, i
   const int log_mp = a.log_m - __ffs(C) + 1;
   Cx* zb = sc + Mp;  // Z for this CTA's k1 slice: [k2][k1 - r slice]
   const int slice = Mp / C;
-  // z[m] = x[2m] + i x[2m + 1] belongs to CTA m mod C.  Each CTA reads a contiguous slice of the
-  // row and hands its samples out through distributed shared memory: read where they belong,
-  // every C-th sample, a warp's load would touch 32 sectors for 16 bytes of each, over every
-  // node group (five modes and groups, FP32: 32.1 -> 28.6 us an evaluation).  A row of one group
-  // is read where it belongs: there the cluster's two barriers cost more (one mode: +2 %).
-  const bool hand_out = row < a.n_partial_rows && a.n_groups > 1;  // uniform over the cluster
+  // z[m] = x[2m] + i x[2m + 1] belongs to CTA m mod C.  Of a long sum (the node groups' rows of this
+  // row, a MB of them at least) each CTA reads a contiguous slice and hands its samples out through
+  // distributed shared memory: read where they belong, every C-th sample, a warp's load touches 32
+  // sectors for 16 bytes of each.  Eight modes and groups of 32 768, FP64 (2 MB): 115 -> 110 us an
+  // evaluation; at 1 MB, both forms and types, within 2 %; below it the cluster's two barriers cost
+  // more (four of 8 192: 17.6 -> 18.6 us), and there every CTA reads its own samples.
+  const bool hand_out = row < a.n_partial_rows && a.n_groups > 1 &&  // uniform over the cluster
+                        (size_t)a.n_groups * a.n_to * sizeof(R) >= ((size_t)1 << 20);
   Cx* home = sc;  // of every sample this thread reads
   if (hand_out) {
     home = cluster.map_shared_rank(sc, (unsigned)threadIdx.x % C);
